@@ -566,7 +566,6 @@ int igr_pattern_route(igr_ctx *c, int n, const int32_t *node_off, const int32_t 
         c->h.alloc(1);
         cuda_check(cudaMemsetAsync(c->h.p, 0, sizeof(int), c->s), "memset");
         tb.queue = c->h.p;
-        tb.tile = kPatternNodeTile;
         launch_pattern_route(g, tb, stamp, c->s);
         cuda_check(cudaMemcpyAsync(routes_out, c->routes.p, ext * 4, cudaMemcpyDeviceToHost, c->s), "D2H");
         sync_check(c);

@@ -72,6 +72,14 @@ void launch_wire_commit(const GridDev &g, int stamp, bool only_dirty, cudaStream
 // track; refresh = false only commits and marks the costs dirty.
 void launch_commit_refresh(const GridDev &g, int *vcnt, int stamp, bool refresh, cudaStream_t s);
 
+// What a checking kernel found before a tree DP launch that the host does not
+// wait in between for: the DP does nothing when a status bit is set or more
+// nodes need scratch than there is (TreeBatchDev::scratch_nodes).
+struct PatternGate {
+    int status = 0, pad = 0;
+    unsigned long long big_nodes = 0;
+};
+
 struct TreeBatchDev {
     const int *net_ids;      // [n] routing-net id of each net of the batch
     const int *node_off;     // [routing nets+1] node offset of each net id (into nodes/par)
@@ -86,14 +94,13 @@ struct TreeBatchDev {
     int n;
     const int *order = nullptr;  // [n] positions into net_ids in processing order (null: 0..n-1)
     int *queue = nullptr;        // work counter of this launch (zero before the launch)
-    int lanes_per_net = 32;      // 16 or 32
-    int tile = 16;               // nodes kept on chip: 6, 16, 32, or 1 (all in scratch)
+    const PatternGate *gate = nullptr;  // optional: checks the launch depends on
     int *vcnt = nullptr;         // non-null: count via crossings per cell here (and the via
                                  // count in stats[1]) for launch_commit_refresh
 };
-// scratch per node of a net kept in global memory: 45 range costs (doubles),
-// then 8 via-column costs (floats), 45 backtrace codes (shorts, padded to 23
-// ints), the chosen range and 4 decoded position/parent ints
+// scratch per node of a net of more than kPatternNodeTile nodes: 45 range costs
+// (doubles), then 8 unused ints, 45 backtrace codes (shorts, padded to 23 ints),
+// the chosen range and 4 unused ints
 constexpr int kPatternScratchD = 45, kPatternScratchI = 8 + 23 + 1 + 4;
 // doubles of scratch needed for `nodes` nodes of nets kept in global memory
 inline int64_t pattern_scratch_doubles(int64_t nodes) {

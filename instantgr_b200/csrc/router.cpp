@@ -888,16 +888,11 @@ void Router::emit_phase1(const std::vector<int> &batch_off, const std::vector<in
             tb.vcnt = split ? nullptr : d_vcnt.p;
             cudaStream_t cs = s;
             if (batched) {
-                tb.tile = c == 0 ? 32 : (c == 1 ? kPatternNodeTile : 6);
-                tb.lanes_per_net = tune.lanes[c];
                 if (c != 1) {
                     cs = s_cls[c == 0 ? 0 : 1];
                     cuda_check(cudaStreamWaitEvent(cs, ev_fork, 0), "fork");
                     forked[c] = true;
                 }
-            } else {
-                tb.tile = kPatternNodeTile;  // nets beyond the tile use global scratch in the same launch
-                tb.lanes_per_net = 32;  // 16 lanes: 3.16 -> 3.86 ms per c1 route
             }
             launch_pattern_route(go.g, tb, stamp, cs);
             st.launches += 1;
@@ -986,9 +981,9 @@ void Router::phase1() {
 }
 
 // Autotuner of the batched form: picks the node count that separates small
-// from medium nets and the lanes per net of each size class by timing the
-// phase-1 batch loop of this design once per candidate (the routes are the
-// same for every candidate).  Results are cached per grid and net count in
+// from medium nets, or one class of all nets, by timing the phase-1 batch loop
+// of this design once per candidate (the routes are the same for every
+// candidate).  Results are cached per grid and net count in
 // $IGR_TUNE_CACHE (default ~/.cache/instantgr_b200/tune.txt).
 static std::string tune_cache_path() {
     if (const char *p = std::getenv("IGR_TUNE_CACHE")) return p;
@@ -1011,7 +1006,7 @@ void Router::autotune(int nb) {
                 auto lanes_ok = [](int l) { return l == 16 || l == 32; };
                 if (std::string(k2) == key && (cl == 1 || cl == 3) && sp >= 1 && sp <= 6 && lanes_ok(l0) &&
                     lanes_ok(l1) && lanes_ok(l2)) {
-                    tune.classes = cl; tune.split = sp; tune.lanes[0] = l0; tune.lanes[1] = l1; tune.lanes[2] = l2;
+                    tune.classes = cl; tune.split = sp;
                     tuned = true;
                 }
             }
@@ -1020,18 +1015,12 @@ void Router::autotune(int nb) {
         if (tuned) return;
     }
     std::vector<Tune> cands;
-    for (int lm : {32, 16}) {
+    cands.push_back(Tune());
+    for (int sp : {3, 4, 6}) {
         Tune t;
-        t.classes = 1; t.lanes[1] = lm;
+        t.classes = 3; t.split = sp;
         cands.push_back(t);
     }
-    for (int sp : {3, 4, 6})
-        for (int lm : {16, 32})
-            for (int ls : {16, 32}) {
-                Tune t;
-                t.classes = 3; t.split = sp; t.lanes[0] = 32; t.lanes[1] = lm; t.lanes[2] = ls;
-                cands.push_back(t);
-            }
     Tune best = tune;
     float best_ms = 1e30f;
     std::vector<int> batch_off, class_off;
@@ -1061,8 +1050,7 @@ void Router::autotune(int nb) {
     go.reset_demand(s);
     if (go.check_error(s)) throw Error(ERR_STATE, "device error while autotuning");
     if (verbose)
-        std::fprintf(stderr, "[igr] autotune: %d classes, split %d, lanes %d/%d/%d (%.2f ms)\n", tune.classes,
-                     tune.split, tune.lanes[0], tune.lanes[1], tune.lanes[2], best_ms);
+        std::fprintf(stderr, "[igr] autotune: %d classes, split %d (%.2f ms)\n", tune.classes, tune.split, best_ms);
     const size_t slash = path.rfind('/');
     if (slash != std::string::npos) {
         const std::string dir = path.substr(0, slash);
@@ -1070,8 +1058,7 @@ void Router::autotune(int nb) {
             if (i == dir.size() || dir[i] == '/') (void)mkdir(dir.substr(0, i).c_str(), 0755);
     }
     if (FILE *f = std::fopen(path.c_str(), "a")) {
-        std::fprintf(f, "%s %d %d %d %d %d\n", key, tune.classes, tune.split, tune.lanes[0], tune.lanes[1],
-                     tune.lanes[2]);
+        std::fprintf(f, "%s %d %d 32 32 32\n", key, tune.classes, tune.split);  // 32 lanes per net in each class
         std::fclose(f);
     }
 }

@@ -263,12 +263,11 @@ struct Router {
     int64_t setup_h2d = 0;              // host-to-device bytes of the device setup
     DevBuf<int> d_ids, d_all_ids, of_sum, d_perm, d_map, d_bat, d_act, d_flags, d_queue;
     DevBuf<int> d_rev_off, d_rev_cnt, d_rev, d_snap, d_dirty, d_part;  // colouring: claimers per cell, round-0 map
-    // launch shape of the tree DP per size class (large, medium, small) and the
-    // node count that separates small from medium nets (autotuned, see tune.cpp)
+    // launches of the tree DP per batch and the node count that separates small
+    // from medium nets (autotuned)
     struct Tune {
         int classes = 1;  // 1: one DP launch per batch (largest nets first); 3: large/medium/small launches
         int split = 6;
-        int lanes[3] = {32, 32, 16};
     } tune;
     bool tuned = false;
     DevBuf<int64_t> d_route_off1;
