@@ -855,7 +855,7 @@ void Router::plan_phase1(int nb, std::vector<int> &batch_off, std::vector<int> &
 void Router::emit_phase1(const std::vector<int> &batch_off, const std::vector<int> &class_off, bool timed) {
     const int nb = (int)batch_off.size() - 1;
     // the fused per-track commit holds tracks of up to kMaxFusedTrackCells cells
-    const bool split = split || std::max(go.g.X, go.g.Y) > kMaxFusedTrackCells;
+    const bool split = split_commit || std::max(go.g.X, go.g.Y) > kMaxFusedTrackCells;
     cuda_check(cudaMemsetAsync(d_queue.p, 0, (3 * (size_t)nb + 1) * sizeof(int), s), "memset");
     for (int bi = 0; bi < nb; bi++) {
         const int off = batch_off[bi], n = batch_off[bi + 1] - off;
