@@ -31,9 +31,10 @@ struct ConvSpec {
 void launch_conv_fwd(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __nv_bfloat16 *W, const float *bias,
                      __nv_bfloat16 *Y, float *Y32, int *err, cudaStream_t s);
 // Input gradient: dXpre[T][hin][win][cin] = (conv^T dY) * (Aprev > 0) (Aprev null: no mask);
-// WT = weights as [cin][9][cout].
+// WT = weights as [cin][9][cout].  db (optional) += sum of dXpre over pixels, [cin]: the
+// bias gradient of the layer before.
 void launch_conv_dgrad(const ConvSpec &c, int T, const __nv_bfloat16 *dY, const __nv_bfloat16 *WT,
-                       const __nv_bfloat16 *Aprev, __nv_bfloat16 *dXpre, int *err, cudaStream_t s);
+                       const __nv_bfloat16 *Aprev, __nv_bfloat16 *dXpre, float *db, int *err, cudaStream_t s);
 // Weight gradient, accumulated: dWT[9*cin][cout] += sum over output pixels (f32 atomics).
 void launch_conv_wgrad(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __nv_bfloat16 *dY, float *dWT,
                        int *err, cudaStream_t s);

@@ -208,8 +208,9 @@ double SeedModel::backward(int T, double *mae) {
     for (int i = kSeedConvs - 1; i >= 0; i--) {
         const __nv_bfloat16 *X = i == 0 ? x0.p : act[i - 1].p;
         launch_conv_wgrad(spec[i], T, X, grad[i].p, dWT[i].p, err.p, s);
-        launch_bias_grad(spec[i], T, grad[i].p, db[i].p, s);
-        if (i > 0) launch_conv_dgrad(spec[i], T, grad[i].p, WT[i].p, act[i - 1].p, grad[i - 1].p, err.p, s);
+        if (i == kSeedConvs - 1) launch_bias_grad(spec[i], T, grad[i].p, db[i].p, s);
+        if (i > 0)
+            launch_conv_dgrad(spec[i], T, grad[i].p, WT[i].p, act[i - 1].p, grad[i - 1].p, db[i - 1].p, err.p, s);
     }
     for (int i = 0; i < kSeedConvs; i++) launch_seed_grad_layout(kCin[i], kCout[i], dWT[i].p, dW[i].p, s);
     double h[2] = {0, 0};

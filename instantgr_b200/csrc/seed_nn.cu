@@ -35,12 +35,6 @@ constexpr unsigned long long kWaitNs = 2000000000ull;
 template <int BN>
 constexpr size_t stage_bytes() { return (size_t)4 * (128 + BN) * 16 * 2; }
 
-__device__ __forceinline__ void put8(__nv_bfloat16 *stage, int r, int kk, uint4 v) {
-    *reinterpret_cast<uint4 *>(stage + (kk >> 4) * (128 * 16) + umma::sub_idx(r, kk & 15)) = v;
-}
-__device__ __forceinline__ void put8b(__nv_bfloat16 *stage, int bn, int r, int kk, uint4 v) {
-    *reinterpret_cast<uint4 *>(stage + (kk >> 4) * (bn * 16) + umma::sub_idx(r, kk & 15)) = v;
-}
 __device__ __forceinline__ void put1(__nv_bfloat16 *stage, int rows, int r, int kk, __nv_bfloat16 v) {
     stage[(kk >> 4) * (rows * 16) + umma::sub_idx(r, kk & 15)] = v;
 }
@@ -64,132 +58,6 @@ __device__ __forceinline__ bool in_pos(const ConvSpec &c, int oy, int ox, int dy
     }
     return iy >= 0 && ix >= 0 && iy < c.hin && ix < c.win;
 }
-
-struct FwdOp {
-    ConvSpec c;
-    const __nv_bfloat16 *X, *W;
-    const float *bias;
-    __nv_bfloat16 *Y;
-    float *Y32;
-    int M, K;
-    __device__ void load_a(__nv_bfloat16 *sa, int m0, int k0, int ke) const {
-        const int tid = threadIdx.x, kc = tid & 7, k = k0 + kc * 8;
-        const int lc = ilog2(c.cin);
-        const int tap = k >> lc, ci = k & (c.cin - 1), dy = tap / 3, dx = tap - 3 * (tap / 3);
-        const int hw = c.hout * c.wout;
-        // every load of the stage in flight before the first store
-        uint4 v[kRowPasses];
-#pragma unroll
-        for (int it = 0; it < kRowPasses; it++) {
-            const int m = m0 + (tid >> 3) + 16 * it;
-            v[it] = make_uint4(0, 0, 0, 0);
-            if (m < M && k < ke) {
-                const int t = m / hw, rem = m - t * hw, oy = rem / c.wout, ox = rem - oy * c.wout;
-                int iy, ix;
-                if (in_pos(c, oy, ox, dy, dx, iy, ix))
-                    v[it] = *reinterpret_cast<const uint4 *>(X + (((size_t)t * c.hin + iy) * c.win + ix) * c.cin + ci);
-            }
-        }
-#pragma unroll
-        for (int it = 0; it < kRowPasses; it++) put8(sa, (tid >> 3) + 16 * it, kc * 8, v[it]);
-    }
-    template <int BN>
-    __device__ void load_b(__nv_bfloat16 *sb, int n0, int k0, int ke) const {
-        uint4 v[BN / 16];
-#pragma unroll
-        for (int it = 0; it < BN / 16; it++) {
-            const int q = threadIdx.x + 128 * it, r = q >> 3, kc = q & 7, k = k0 + kc * 8, n = n0 + r;
-            v[it] = make_uint4(0, 0, 0, 0);
-            if (n < c.cout && k < ke) v[it] = *reinterpret_cast<const uint4 *>(W + (size_t)n * K + k);
-        }
-#pragma unroll
-        for (int it = 0; it < BN / 16; it++) {
-            const int q = threadIdx.x + 128 * it;
-            put8b(sb, BN, q >> 3, (q & 7) * 8, v[it]);
-        }
-    }
-    __device__ void store(int row, int n0, const float *v) const {
-        if (row >= M || n0 >= c.cout) return;
-        __align__(16) __nv_bfloat16 o[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            float x = v[j] + bias[n0 + j];
-            if (c.relu) x = fmaxf(x, 0.f);
-            o[j] = __float2bfloat16(x);
-            if (Y32) Y32[(size_t)row * c.cout + n0 + j] = x;
-        }
-        *reinterpret_cast<uint4 *>(Y + (size_t)row * c.cout + n0) = *reinterpret_cast<const uint4 *>(o);
-    }
-};
-
-struct DgradOp {
-    ConvSpec c;
-    const __nv_bfloat16 *dY, *WT, *Aprev;
-    __nv_bfloat16 *dX;
-    int M, K;
-    __device__ void load_a(__nv_bfloat16 *sa, int m0, int k0, int ke) const {
-        const int tid = threadIdx.x, kc = tid & 7, k = k0 + kc * 8;
-        const int lc = ilog2(c.cout), per = 9 * c.cout;
-        const int sub = k / per, rem = k - sub * per;
-        const int tap = rem >> lc, co = rem & (c.cout - 1), dy = tap / 3, dx = tap - 3 * (tap / 3);
-        const int hw = c.hin * c.win;
-        uint4 v[kRowPasses];
-#pragma unroll
-        for (int it = 0; it < kRowPasses; it++) {
-            const int m = m0 + (tid >> 3) + 16 * it;
-            v[it] = make_uint4(0, 0, 0, 0);
-            if (m < M && k < ke) {
-                const int t = m / hw, q = m - t * hw, iy = q / c.win, ix = q - iy * c.win;
-                int oy, ox;
-                bool ok;
-                if (c.mode == 1) {
-                    const int ny = iy + 1 - dy, nx = ix + 1 - dx;
-                    ok = ny >= 0 && nx >= 0 && !(ny & 1) && !(nx & 1);
-                    oy = ny >> 1;
-                    ox = nx >> 1;
-                } else if (c.mode == 2) {
-                    oy = 2 * iy + (sub >> 1) + 1 - dy;
-                    ox = 2 * ix + (sub & 1) + 1 - dx;
-                    ok = true;
-                } else {
-                    oy = iy + 1 - dy;
-                    ox = ix + 1 - dx;
-                    ok = true;
-                }
-                ok = ok && oy >= 0 && ox >= 0 && oy < c.hout && ox < c.wout;
-                if (ok)
-                    v[it] = *reinterpret_cast<const uint4 *>(dY + (((size_t)t * c.hout + oy) * c.wout + ox) * c.cout + co);
-            }
-        }
-#pragma unroll
-        for (int it = 0; it < kRowPasses; it++) put8(sa, (tid >> 3) + 16 * it, kc * 8, v[it]);
-    }
-    template <int BN>
-    __device__ void load_b(__nv_bfloat16 *sb, int n0, int k0, int ke) const {
-        const int per = 9 * c.cout;
-        uint4 v[BN / 16];
-#pragma unroll
-        for (int it = 0; it < BN / 16; it++) {
-            const int q = threadIdx.x + 128 * it, r = q >> 3, kc = q & 7, k = k0 + kc * 8, n = n0 + r;
-            v[it] = make_uint4(0, 0, 0, 0);
-            if (n < c.cin && k < ke) v[it] = *reinterpret_cast<const uint4 *>(WT + (size_t)n * per + (k % per));
-        }
-#pragma unroll
-        for (int it = 0; it < BN / 16; it++) {
-            const int q = threadIdx.x + 128 * it;
-            put8b(sb, BN, q >> 3, (q & 7) * 8, v[it]);
-        }
-    }
-    __device__ void store(int row, int n0, const float *v) const {
-        if (row >= M || n0 >= c.cin) return;
-        __align__(16) __nv_bfloat16 o[8];
-        __align__(16) __nv_bfloat16 a[8];
-        if (Aprev) *reinterpret_cast<uint4 *>(a) = *reinterpret_cast<const uint4 *>(Aprev + (size_t)row * c.cin + n0);
-#pragma unroll
-        for (int j = 0; j < 8; j++) o[j] = __float2bfloat16((!Aprev || __bfloat162float(a[j]) > 0.f) ? v[j] : 0.f);
-        *reinterpret_cast<uint4 *>(dX + (size_t)row * c.cin + n0) = *reinterpret_cast<const uint4 *>(o);
-    }
-};
 
 struct WgradOp {
     ConvSpec c;
@@ -491,18 +359,6 @@ __global__ void seed_grad_layout_kernel(int cin, int cout, const float *dWT, flo
 int blocks_for(long long n) { return (int)std::max<long long>(1, std::min<long long>(148 * 8, (n + 255) / 256)); }
 
 }  // namespace
-
-void launch_conv_fwd(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __nv_bfloat16 *W, const float *bias,
-                     __nv_bfloat16 *Y, float *Y32, int *err, cudaStream_t s) {
-    FwdOp op{c, X, W, bias, Y, Y32, T * c.hout * c.wout, 9 * c.cin};
-    launch_by_n(op, c.cout, 0, err, s);
-}
-
-void launch_conv_dgrad(const ConvSpec &c, int T, const __nv_bfloat16 *dY, const __nv_bfloat16 *WT,
-                       const __nv_bfloat16 *Aprev, __nv_bfloat16 *dXpre, int *err, cudaStream_t s) {
-    DgradOp op{c, dY, WT, Aprev, dXpre, T * c.hin * c.win, (c.mode == 2 ? 4 : 1) * 9 * c.cout};
-    launch_by_n(op, c.cin, 0, err, s);
-}
 
 void launch_conv_wgrad(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __nv_bfloat16 *dY, float *dWT,
                        int *err, cudaStream_t s) {
