@@ -1,7 +1,7 @@
-// Convolutions of the learned congestion seed and their input gradients as
-// implicit GEMMs on the tcgen05 tensor cores.
+// Convolutions of the learned congestion seed and their gradients as implicit
+// GEMMs on the tcgen05 tensor cores.
 //
-// All of them multiply rows = output pixels by columns = output channels over
+// The forward convolutions and the input gradients multiply rows = output pixels by columns = output channels over
 // K = taps x input channels.  A tap only shifts which source pixel a row reads,
 // so a source tile is brought into shared memory once, with the pixels around
 // it, and every tap reads it through a descriptor of another start address: the
@@ -243,10 +243,12 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
                 const int x = G::fine ? 2 * (x0 + c) + (j & 1) : x0 + c + 8 * j;
                 in = y < p.oh && x < p.ow;
                 at = in ? (((size_t)img * p.oh + y) * p.ow + x) * N : 0;
-                if constexpr (GRAD)
-                    if (p.mask)
+                if constexpr (GRAD) {
+                    if (p.mask) {
 #pragma unroll
                         for (int i = 0; i < N / 8; i++) m[i] = reinterpret_cast<const uint4 *>(p.mask + at)[i];
+                    }
+                }
             };
             pixel(0);
             ok = umma::mbar_wait(&tfull[s], (it >> 1) & 1, p.wait_ns, &quit);
@@ -311,8 +313,8 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
             umma::fence_before();
             umma::mbar_arrive(&tempty[s]);
         }
-        if constexpr (GRAD)
-            if (p.db && ok)
+        if constexpr (GRAD) {
+            if (p.db && ok) {
 #pragma unroll
                 for (int n = 0; n < N; n++) {
                     float v = sum[n];
@@ -320,6 +322,8 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
                     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
                     if (lane == 0 && mine > 0) atomicAdd(p.db + n, v);
                 }
+            }
+        }
     }
     umma::fence_before();
     if (__syncthreads_and(ok) == 0 && tid == 0) set_error(p.err, ERR_TIMEOUT);
@@ -346,6 +350,267 @@ void launch(ConvArgs a, int T, int gh, int gw, cudaStream_t s) {
     a.probe = test_hooks().mbar_probe.load();
     const int blocks = std::min(a.tiles, ks.sms * std::min(ks.blocks_per_sm, per_sm));
     kernel<<<blocks, kConvThreads, smem, s>>>(a);
+}
+
+// ---------------------------------------------------------------- weight gradients
+//
+// dW[tap][ci][co] = sum over pixels of X[pixel + tap][ci] dY[pixel][co]: K is the
+// pixels, so both operands are MN-major, and the planes of 8 channels serve
+// again: 16 pixels of a tile row are the two K groups of an MMA.  A tile lies
+// [row][plane][pixel], so that an operand of 128 rows, or of N columns, covers
+// several tile rows of channels: A takes 128 / CA rows of its tensor, B the rows
+// of the other one that any of them meets under a tap, and one MMA makes the
+// products of all these row pairs for one horizontal shift.  The tap of a pair is
+// the difference of its rows; pairs further apart are not read out.  All of an
+// SM's sums stay in TMEM over its tiles (at most 512 columns) and go to memory
+// once, by f32 additions.
+//
+// wSame: both tensors at one resolution; A is dY, or X where it has more
+// channels.  wUp2 (X at half the resolution of dY): A is X, B the pixels of dY of
+// one row parity (a block's) and both column parities; nearest upsampling gives
+// the taps that read the same X pixel the same product, which is added to each.
+// wStride2 (X at twice the resolution of dY): A is dY, B the four parities of X.
+// Bound by the operand reads from shared memory (8 KB for 128 x 128 x 16) and
+// the copies of the tiles; transposing both operands through registers element
+// by element, as the kernel before it did, took 3.62 ms for 16 tiles of 288 x 288
+// (now 0.38 ms: 51 and 61 us for the two layers at full resolution, 52 for the
+// strided one and for each of the 64-channel layers, 110 for the upsampled one).
+enum WKind { wSame, wUp2, wStride2 };
+
+template <WKind K, bool AX, int CA, int CB, int CBALL>
+struct WGeo {
+    static constexpr int arows = 128 / CA;               // rows of A in an MMA
+    static constexpr int rows = K == wStride2 ? 8 : 16;  // tile rows of A
+    static constexpr int ach = CA / 8, bch = CB / 8;
+    static constexpr int parts = K == wSame ? 1 : K == wUp2 ? 2 : 4;  // parity classes of B
+    static constexpr int brows = K == wStride2 ? rows + 1 : rows + 2;
+    static constexpr int bcols = K == wStride2 ? 17 : 18;
+    static constexpr int apitch = 17, bpitch = bcols | 1;  // odd: the copies meet no bank conflict
+    static constexpr int part = brows * bch * bpitch * 16;
+    static constexpr int abytes = rows * ach * apitch * 16;
+    static constexpr int bytes = (abytes + parts * part + 127) / 128 * 128;
+    static constexpr int bufs = K == wUp2 ? 2 : 3;
+    static constexpr int smem = bufs * bytes;
+    // columns of TMEM: one MMA's N per horizontal shift (and row parity)
+    static constexpr int n = K == wSame ? (arows + 2) * CB : 3 * CB;
+    static constexpr int shifts = K == wUp2 ? 4 : 3;
+    static constexpr int columns = shifts * n + (K == wStride2 ? shifts * 2 * CB : 0);
+    static_assert(columns <= 512 && n % 16 == 0 && n <= 256, "the sums of an SM");
+};
+
+struct WgradArgs {
+    const __nv_bfloat16 *A, *B;  // channels-last; CA and CBALL channels
+    int ah, aw, bh, bw;
+    int tiles, tx, ty;
+    float *dWT;                  // [9][cin][cout]
+    int cin, cout;
+    int *err;
+    unsigned long long wait_ns;
+    int probe;
+};
+
+__device__ __forceinline__ void add4(float *p, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+template <WKind K, bool AX, int CA, int CB, int CBALL>
+__global__ void __launch_bounds__(kConvThreads, 1) wgrad_kernel(const WgradArgs p) {
+    using G = WGeo<K, AX, CA, CB, CBALL>;
+    extern __shared__ __align__(128) uint8_t sm[];
+    __shared__ __align__(8) uint64_t full[G::bufs], empty[G::bufs], done;
+    __shared__ uint32_t tbase;
+    __shared__ volatile int quit;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int half = blockIdx.y;  // wSame: which CB channels of B; wUp2: row parity of dY
+    if (warp == 0) umma::tmem_alloc(&tbase, 512);
+    if (tid == 0) {
+        quit = 0;
+        for (int i = 0; i < G::bufs; i++) {
+            umma::mbar_init(&full[i], 256);
+            umma::mbar_init(&empty[i]);
+        }
+        umma::mbar_init(&done);
+        umma::mbar_init_fence();
+    }
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const uint32_t tmem = tbase;
+    bool ok = true;
+    if (p.probe) {  // test hook: a wait on a phase that nothing completes, before any MMA is issued
+        if (tid == 0) ok = umma::mbar_wait(&done, 0, p.wait_ns);
+        ok = __syncthreads_and(ok) != 0;
+    }
+    const int per_image = p.tx * p.ty;
+    const int mine = ok && (int)blockIdx.x < p.tiles ? (p.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    if (warp < 8) {
+        for (int it = 0; it < mine; it++) {
+            const int b = it % G::bufs;
+            if (it >= G::bufs) ok = umma::mbar_wait(&empty[b], (it / G::bufs - 1) & 1, p.wait_ns, &quit);
+            if (!ok) break;
+            const int t = blockIdx.x + it * gridDim.x, img = t / per_image, rem = t - img * per_image;
+            const int y0 = rem / p.tx * G::rows, x0 = (rem - rem / p.tx * p.tx) * 16;
+            const uint32_t dst = umma::smem_u32(sm) + b * G::bytes;
+            const __nv_bfloat16 *A = p.A + (size_t)img * p.ah * p.aw * CA;
+#pragma unroll 4
+            for (int q = tid; q < G::rows * 16 * G::ach; q += 256) {
+                const int ch = q % G::ach, px = q / G::ach, r = px >> 4, c = px & 15;
+                const int y = y0 + r, x = x0 + c;
+                const bool in = y < p.ah && x < p.aw;
+                umma::copy16(dst + ((r * G::ach + ch) * G::apitch + c) * 16,
+                             A + (in ? ((size_t)y * p.aw + x) * CA + ch * 8 : 0), in);
+            }
+            const __nv_bfloat16 *B = p.B + (size_t)img * p.bh * p.bw * CBALL + (K == wSame ? half * CB : 0);
+#pragma unroll 4
+            for (int q = tid; q < G::parts * G::brows * G::bcols * G::bch; q += 256) {
+                const int ch = q % G::bch, px = q / G::bch, part = px / (G::brows * G::bcols);
+                const int rc = px - part * (G::brows * G::bcols), r = rc / G::bcols, c = rc - r * G::bcols;
+                int y = y0 - 1 + r, x = x0 - 1 + c;
+                if (K == wUp2) {  // part: column parity
+                    y = 2 * y + half;
+                    x = 2 * x + part;
+                } else if (K == wStride2) {  // part: row parity, column parity
+                    y = 2 * y + (part >> 1);
+                    x = 2 * x + (part & 1);
+                }
+                const bool in = (unsigned)y < (unsigned)p.bh && (unsigned)x < (unsigned)p.bw;
+                umma::copy16(dst + G::abytes + part * G::part + ((r * G::bch + ch) * G::bpitch + c) * 16,
+                             B + (in ? ((size_t)y * p.bw + x) * CBALL + ch * 8 : 0), in);
+            }
+            umma::copy_commit();
+            if (it > 0) {
+                umma::copy_wait<1>();
+                umma::fence_async_smem();
+                umma::mbar_arrive(&full[(it - 1) % G::bufs]);
+            }
+        }
+        umma::copy_wait<0>();
+        umma::fence_async_smem();
+        if (ok && mine > 0) umma::mbar_arrive(&full[(mine - 1) % G::bufs]);
+    } else if (lane == 0) {
+        constexpr uint32_t idesc = umma::idesc_bf16_mn(128, G::n);
+        int issued = 0;
+        for (int it = 0; it < mine; it++) {
+            const int b = it % G::bufs;
+            ok = umma::mbar_wait(&full[b], (it / G::bufs) & 1, p.wait_ns, &quit);
+            if (!ok) break;
+            umma::fence_after();
+            const uint32_t base = umma::smem_u32(sm) + b * G::bytes;
+            const uint64_t da = umma::smem_desc(base, 128, G::apitch * 16);
+            const uint64_t db = umma::smem_desc(base + G::abytes, 128, G::bpitch * 16);
+            // start of row r, column c of part q of B
+            auto at = [](int q, int r, int c) { return (uint64_t)((q * G::part + (r * G::bch * G::bpitch + c) * 16) >> 4); };
+            for (int g = 0; g < G::rows; g += G::arows) {
+                const uint64_t a = da + (uint64_t)(g * G::ach * G::apitch);
+                const bool acc = it > 0 || g > 0;
+                if (K == wSame) {
+#pragma unroll
+                    for (int e = 0; e < 3; e++)
+                        umma::mma_bf16(tmem + e * G::n, a, db + at(0, g, e), idesc, acc);
+                } else if (K == wUp2) {
+#pragma unroll
+                    for (int e = 0; e < 4; e++)  // column parity e >> 1, X column minus dY column - 1 + (e >> 1) + (e & 1)
+                        umma::mma_bf16(tmem + e * G::n, a,
+                                       db + at(e >> 1, g + 1 - half, 2 - (e >> 1) - (e & 1)), idesc, acc);
+                } else {
+                    constexpr uint32_t ieven = umma::idesc_bf16_mn(128, 2 * CB);
+#pragma unroll
+                    for (int dx = 0; dx < 3; dx++) {
+                        const int qx = dx == 1 ? 0 : 1, c = dx == 0 ? 0 : 1;
+                        umma::mma_bf16(tmem + dx * G::n, a, db + at(2 + qx, g, c), idesc, acc);
+                        umma::mma_bf16(tmem + 3 * G::n + dx * 2 * CB, a, db + at(qx, g + 1, c), ieven, acc);
+                    }
+                }
+            }
+            umma::mma_commit(&empty[b]);
+            issued = it + 1;
+        }
+        if (issued > 0) {
+            umma::mma_commit(&done);
+            if (!umma::mbar_wait(&done, 0, kDrainNs)) ok = false;
+        }
+    }
+    umma::fence_before();
+    const bool good = __syncthreads_and(ok) != 0;
+    umma::fence_after();
+    if (good && mine > 0 && warp < 4) {
+        const int a = tid / CA, ca = tid % CA;  // row and channel of A
+        auto place = [&](int ty, int tx, int cb) {
+            const int ci = AX || K == wUp2 ? ca : (K == wSame ? half * CB : 0) + cb;
+            const int co = AX || K == wUp2 ? cb : ca;
+            return p.dWT + ((size_t)(ty * 3 + tx) * p.cin + ci) * p.cout + co;
+        };
+        for (int n0 = 0; n0 < G::columns; n0 += 16) {
+            uint32_t v[16];
+            umma::tmem_ld(tmem + ((uint32_t)(warp * 32) << 16) + n0, v);
+            umma::tmem_wait();
+            const bool even = K == wStride2 && n0 >= 3 * G::n;
+            const int e = even ? (n0 - 3 * G::n) / (2 * CB) : n0 / G::n;
+            const int left = even ? n0 - 3 * G::n - e * 2 * CB : n0 - e * G::n;
+            const int b = left / CB, cb = left - b * CB;
+            // the taps this pair of rows and this shift belong to
+            int ty0 = 0, ty1 = -1, tx0 = 0, tx1 = -1;
+            if (K == wSame) {
+                const int ey = b - a;
+                if (ey >= 0 && ey <= 2) ty0 = ty1 = AX ? 2 - ey : ey;
+                tx0 = tx1 = AX ? 2 - e : e;
+            } else if (K == wUp2) {
+                // X pixel minus dY pixel at half resolution: parity 0: -1 (tap 0), 0 (taps 1, 2);
+                // parity 1: 0 (taps 0, 1), 1 (tap 2)
+                const int oy = a - b + half, ox = -1 + (e >> 1) + (e & 1), px = e >> 1;
+                if (half == 0 && oy == -1) ty0 = ty1 = 0;
+                if (half == 0 && oy == 0) { ty0 = 1; ty1 = 2; }
+                if (half == 1 && oy == 0) { ty0 = 0; ty1 = 1; }
+                if (half == 1 && oy == 1) ty0 = ty1 = 2;
+                if (px == 0 && ox == -1) tx0 = tx1 = 0;
+                if (px == 0 && ox == 0) { tx0 = 1; tx1 = 2; }
+                if (px == 1 && ox == 0) { tx0 = 0; tx1 = 1; }
+                if (px == 1 && ox == 1) tx0 = tx1 = 2;
+            } else {
+                if (even) {
+                    if (b == a) ty0 = ty1 = 1;
+                } else {
+                    if (b == a) ty0 = ty1 = 0;
+                    if (b == a + 1) ty0 = ty1 = 2;
+                }
+                tx0 = tx1 = e;
+            }
+            for (int ty = ty0; ty <= ty1; ty++)
+                for (int tx = tx0; tx <= tx1; tx++) {
+                    if (AX || K == wUp2) {
+                        float *q = place(ty, tx, cb);
+#pragma unroll
+                        for (int i = 0; i < 16; i += 4)
+                            add4(q + i, __uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]),
+                                 __uint_as_float(v[i + 3]));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; i++) atomicAdd(place(ty, tx, cb + i), __uint_as_float(v[i]));
+                    }
+                }
+        }
+        umma::fence_before();
+    } else if (!good && tid == 0) {
+        set_error(p.err, ERR_TIMEOUT);
+    }
+    __syncthreads();
+    if (warp == 0) umma::tmem_free(tmem, 512);
+}
+
+template <WKind K, bool AX, int CA, int CB, int CBALL>
+void launch_wgrad(WgradArgs a, int T, int halves, cudaStream_t s) {
+    using G = WGeo<K, AX, CA, CB, CBALL>;
+    constexpr int floor_bytes = 228 * 1024 / 2 - 1024 + 16;  // one block holds an SM's TMEM
+    constexpr int smem = G::smem > floor_bytes ? G::smem : floor_bytes;
+    static_assert(smem <= 227 * 1024, "a block's shared memory");
+    const auto kernel = wgrad_kernel<K, AX, CA, CB, CBALL>;
+    const KernelShape ks = kernel_setup((const void *)kernel, kConvThreads, smem);
+    a.ty = (a.ah + G::rows - 1) / G::rows;
+    a.tx = (a.aw + 15) / 16;
+    a.tiles = T * a.ty * a.tx;
+    a.wait_ns = (unsigned long long)test_hooks().wait_ns.load();
+    a.probe = test_hooks().mbar_probe.load();
+    kernel<<<dim3(std::min(a.tiles, ks.sms / halves), halves), kConvThreads, smem, s>>>(a);
 }
 
 [[noreturn]] void no_kernel(const ConvSpec &c) {
@@ -379,6 +644,28 @@ void launch_conv_dgrad(const ConvSpec &c, int T, const __nv_bfloat16 *dY, const 
     else if (key == 3216) launch<kSame, 16, 32, true, 2>(a, T, c.hin, c.win, s);
     else if (key == 13264) launch<kStride2T, 64, 32, true, 2>(a, T, c.hout, c.wout, s);
     else if (key == 26432) launch<kUp2T, 32, 64, true, 1>(a, T, c.hin, c.win, s);
+    else no_kernel(c);
+}
+
+void launch_conv_wgrad(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __nv_bfloat16 *dY, float *dWT,
+                       int *err, cudaStream_t s) {
+    WgradArgs a{};
+    a.dWT = dWT; a.cin = c.cin; a.cout = c.cout; a.err = err;
+    auto of_x = [&](const __nv_bfloat16 *&t, int &h, int &w) { t = X; h = c.hin; w = c.win; };
+    auto of_dy = [&](const __nv_bfloat16 *&t, int &h, int &w) { t = dY; h = c.hout; w = c.wout; };
+    const int key = c.mode * 10000 + c.cin * 100 + c.cout;
+    if (key == 3216 || key == 26432) {  // A is X
+        of_x(a.A, a.ah, a.aw);
+        of_dy(a.B, a.bh, a.bw);
+        if (key == 3216) launch_wgrad<wSame, true, 32, 16, 16>(a, T, 1, s);
+        else launch_wgrad<wUp2, true, 64, 32, 32>(a, T, 2, s);
+        return;
+    }
+    of_dy(a.A, a.ah, a.aw);
+    of_x(a.B, a.bh, a.bw);
+    if (key == 1632) launch_wgrad<wSame, false, 32, 16, 16>(a, T, 1, s);
+    else if (key == 6464) launch_wgrad<wSame, false, 64, 32, 64>(a, T, 2, s);
+    else if (key == 13264) launch_wgrad<wStride2, false, 64, 32, 32>(a, T, 1, s);
     else no_kernel(c);
 }
 

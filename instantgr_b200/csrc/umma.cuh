@@ -4,7 +4,9 @@
 // TMEM loads.  Operand tiles use the canonical layouts without swizzle: core
 // matrices of 8 x 16 bytes (128 contiguous bytes).  K-major: 8 rows of 8 K
 // elements each, the two K halves of a K = 16 step apart by the leading byte
-// offset, groups of 8 rows by the stride byte offset.
+// offset, groups of 8 rows by the stride byte offset.  MN-major: 8 K rows of 8
+// elements along M or N each, groups of 8 K apart by the leading byte offset,
+// groups of 8 elements along M or N by the stride byte offset.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -37,6 +39,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) { return smem_desc
 // kind::f16 instruction descriptor: F32 accumulator, BF16 A and B, both K-major
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// the same with both operands MN-major (the sum runs over the core matrices' rows)
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
+    return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
 
 // one warp: allocate `cols` TMEM columns (power of two >= 32), address into *dst
