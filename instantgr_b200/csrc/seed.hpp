@@ -21,6 +21,19 @@ constexpr int kSeedTile = 256;  // predicted region per tile
 constexpr int kSeedHalo = 16;
 constexpr int kSeedS = kSeedTile + 2 * kSeedHalo;  // 288: tile with halo
 constexpr int kSeedConvs = 6;
+// channels of the convolutions; the parameters of all of them lie end to end,
+// per convolution its weights [cout][9][cin], then its biases
+#ifdef __CUDACC__
+#define IGR_HD __host__ __device__
+#else
+#define IGR_HD
+#endif
+IGR_HD constexpr int seed_cin(int i) { return i == 0 ? 16 : i == 1 || i == 5 ? 32 : 64; }
+IGR_HD constexpr int seed_cout(int i) { return i == 0 || i == 4 ? 32 : i == 5 ? 16 : 64; }
+IGR_HD constexpr int seed_weights(int i) { return 9 * seed_cin(i) * seed_cout(i); }
+IGR_HD constexpr int seed_at(int i) { return i == 0 ? 0 : seed_at(i - 1) + seed_weights(i - 1) + seed_cout(i - 1); }
+IGR_HD constexpr int seed_bias_at(int i) { return seed_at(i) + seed_weights(i); }
+constexpr int kSeedParams = seed_at(kSeedConvs - 1) + seed_weights(kSeedConvs - 1) + seed_cout(kSeedConvs - 1);
 
 // one 3x3 convolution: mode 0 same size, 1 stride 2, 2 nearest upsample x2 then same
 struct ConvSpec {
@@ -38,21 +51,19 @@ void launch_conv_dgrad(const ConvSpec &c, int T, const __nv_bfloat16 *dY, const 
 // Weight gradient, accumulated: dWT[9*cin][cout] += sum over output pixels (f32 atomics).
 void launch_conv_wgrad(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __nv_bfloat16 *dY, float *dWT,
                        int *err, cudaStream_t s);
-// Bias gradient: db[cout] += sum over pixels of dY.
-void launch_bias_grad(const ConvSpec &c, int T, const __nv_bfloat16 *dY, float *db, cudaStream_t s);
 // MSE loss over the central region [halo, S - halo)^2 of each S x S tile and the 10
 // demand channels: dY = 2 (y - t) / count (bf16, zero elsewhere); sums[0] += sum of
-// squared errors, sums[1] += sum of absolute errors (f64).
+// squared errors, sums[1] += sum of absolute errors (f64), db[16] += sum of dY over pixels.
 void launch_seed_loss(int T, int S, int halo, const float *y, const float *target, __nv_bfloat16 *dY, double *sums,
-                      cudaStream_t s);
+                      float *db, cudaStream_t s);
 // Tiles from channels-last maps: out[t][i][j][c] = map_t[(x0_t - halo + i) * Y_t + (y0_t - halo + j)][c]
-// (0 outside the map), for maps of bf16 (features) or bf16 -> f32 (targets).
+// (0 outside the map): bf16 features and, where given, f32 targets from their bf16 pool.
 struct TileRef {
     long long base;  // element offset of the map in the pool (cells x 16 channels)
     int X, Y, x0, y0;
 };
-void launch_gather_tiles(int T, int S, int halo, const TileRef *tiles, const __nv_bfloat16 *pool, __nv_bfloat16 *out16,
-                         float *out32, cudaStream_t s);
+void launch_gather_tiles(int T, int S, int halo, const TileRef *tiles, const __nv_bfloat16 *features,
+                         __nv_bfloat16 *out16, const __nv_bfloat16 *targets, float *out32, cudaStream_t s);
 // Writes the central (S - 2 halo)^2 region of each tile's output y32 into the
 // channels-last prediction map pred [X][Y][16] (cells outside the map skipped).
 void launch_scatter_prediction(int T, int S, int halo, const TileRef *tiles, const float *y32, float *pred,
@@ -72,13 +83,17 @@ void launch_seed_step(int64_t n, float *demand, const float *base, float *cur, f
 void launch_seed_overflow(int X, int Y, int L, const float *pred, const float *cap_ref, float *out, cudaStream_t s);
 // demand[i] += sign * seed[i] over n cells
 void launch_add_demand(int64_t n, float *demand, const float *seed, float sign, cudaStream_t s);
-// Adam step over n parameters (f32 master, gradient, moments), bias-corrected.
-void launch_adam(int n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2, float eps, int t,
-                 cudaStream_t s);
-// Working weights of a convolution from its master copy: W[cout][9][cin], WT[cin][9][cout] (bf16),
-// and the gradient layout conversion dW[cout][9][cin] <- dWT[9*cin][cout].
-void launch_seed_weights(int cin, int cout, const float *Wm, __nv_bfloat16 *W, __nv_bfloat16 *WT, cudaStream_t s);
-void launch_seed_grad_layout(int cin, int cout, const float *dWT, float *dW, cudaStream_t s);
+// Gradient sums as the convolutions leave them (`acc`, kSeedParams floats): each
+// weight block as [9 * cin][cout], biases in their places.
+// Adam step over all parameters P (f32 master, moments), bias-corrected, and the
+// working weights of the updated ones.
+void launch_adam(float *P, float *M, float *V, const float *acc, __nv_bfloat16 *W, __nv_bfloat16 *WT, float lr, float b1,
+                 float b2, float eps, int t, cudaStream_t s);
+// Working weights of all convolutions: per convolution W[cout][9][cin] and
+// WT[cin][9][cout] (bf16) at the offset of its parameters.
+void launch_seed_weights(const float *P, __nv_bfloat16 *W, __nv_bfloat16 *WT, cudaStream_t s);
+// Gradients in the order of the parameters from `acc`.
+void launch_seed_grad_layout(const float *acc, float *G, cudaStream_t s);
 // The 16 input channels of a design ([X][Y][16] bf16, seed_feat.cu) from the
 // resident trees of its n routing nets (positions l*X*Y + x*Y + y, Steiner
 // points at layer g.L), the capacity of file layer 0 (cap0, [x][y]) and the

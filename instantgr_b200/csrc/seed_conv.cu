@@ -314,14 +314,20 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
             umma::mbar_arrive(&tempty[s]);
         }
         if constexpr (GRAD) {
-            if (p.db && ok) {
+            if (p.db && ok && mine > 0) {
+                // sums over the lanes: half of the channels change hands at each step,
+                // until lane l has channels l N / 32 ..
 #pragma unroll
-                for (int n = 0; n < N; n++) {
-                    float v = sum[n];
+                for (int o = 16, half = N / 2; o > 0; o >>= 1, half /= 2) {
+                    const bool up = lane & o;
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                    if (lane == 0 && mine > 0) atomicAdd(p.db + n, v);
+                    for (int n = 0; n < half; n++) {
+                        const float give = up ? sum[n] : sum[n + half];
+                        sum[n] = (up ? sum[n + half] : sum[n]) + __shfl_xor_sync(0xffffffffu, give, o);
+                    }
                 }
+#pragma unroll
+                for (int n = 0; n < N / 32; n++) atomicAdd(p.db + lane * (N / 32) + n, sum[n]);
             }
         }
     }

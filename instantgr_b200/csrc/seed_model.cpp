@@ -31,9 +31,6 @@ double normal(uint64_t &s) {
     return std::sqrt(-2.0 * std::log(u)) * std::cos(6.283185307179586 * v);
 }
 
-const int kCin[kSeedConvs] = {16, 32, 64, 64, 64, 32};
-const int kCout[kSeedConvs] = {32, 64, 64, 64, 32, 16};
-
 }  // namespace
 
 void SeedModel::set_tile(int S_, int halo_) {
@@ -54,70 +51,39 @@ void SeedModel::init(uint64_t seed) {
     if (!s) cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     if (spec[0].cin == 0) set_tile(kSeedS, kSeedHalo);
     uint64_t r = seed * 0x2545F4914F6CDD1Dull + 17;
-    std::vector<float> w;
+    std::vector<float> p(kSeedParams, 0.f);
     for (int i = 0; i < kSeedConvs; i++) {
-        const int n = kCout[i] * 9 * kCin[i];
-        w.assign(n, 0.f);
-        const double sd = std::sqrt(2.0 / (9.0 * (i == 0 ? kSeedFeat : kCin[i]))) * (i == kSeedConvs - 1 ? 0.1 : 1.0);
-        for (int co = 0; co < kCout[i]; co++)
-            for (int k = 0; k < 9 * kCin[i]; k++) {
-                const int ci = k % kCin[i];
+        const int cin = seed_cin(i), cout = seed_cout(i);
+        const double sd = std::sqrt(2.0 / (9.0 * (i == 0 ? kSeedFeat : cin))) * (i == kSeedConvs - 1 ? 0.1 : 1.0);
+        for (int co = 0; co < cout; co++)
+            for (int k = 0; k < 9 * cin; k++) {
+                const int ci = k % cin;
                 const bool used = (i > 0 || ci < kSeedFeat) && (i < kSeedConvs - 1 || co < kSeedLayersOut);
-                w[(size_t)co * 9 * kCin[i] + k] = used ? (float)(normal(r) * sd) : 0.f;
+                p[seed_at(i) + (size_t)co * 9 * cin + k] = used ? (float)(normal(r) * sd) : 0.f;
             }
-        std::vector<float> z(kCout[i], 0.f);
-        set_layer(i, w.data(), z.data());
     }
-    adam_t = 0;
-}
-
-void SeedModel::set_layer(int i, const float *w, const float *b) {
-    const int n = kCout[i] * 9 * kCin[i];
-    Wm[i].upload(w, n, s);
-    bias[i].upload(b, kCout[i], s);
-    W[i].alloc(n);
-    WT[i].alloc(n);
-    for (auto *buf : {&mW[i], &vW[i], &dW[i], &dWT[i]}) {
-        buf->alloc(n);
-        cuda_check(cudaMemsetAsync(buf->p, 0, n * sizeof(float), s), "memset");
-    }
-    for (auto *buf : {&mb[i], &vb[i], &db[i]}) {
-        buf->alloc(kCout[i]);
-        cuda_check(cudaMemsetAsync(buf->p, 0, kCout[i] * sizeof(float), s), "memset");
-    }
-    launch_seed_weights(kCin[i], kCout[i], Wm[i].p, W[i].p, WT[i].p, s);
-    cuda_check(cudaStreamSynchronize(s), "seed weights");
-}
-
-int SeedModel::params() const {
-    int n = 0;
-    for (int i = 0; i < kSeedConvs; i++) n += kCout[i] * 9 * kCin[i] + kCout[i];
-    return n;
+    set_params(p.data(), p.size());
 }
 
 void SeedModel::get_params(std::vector<float> &out) {
-    out.clear();
-    for (int i = 0; i < kSeedConvs; i++) {
-        const int n = kCout[i] * 9 * kCin[i];
-        std::vector<float> w(n), b(kCout[i]);
-        cuda_check(cudaMemcpyAsync(w.data(), Wm[i].p, n * 4, cudaMemcpyDeviceToHost, s), "D2H");
-        cuda_check(cudaMemcpyAsync(b.data(), bias[i].p, kCout[i] * 4, cudaMemcpyDeviceToHost, s), "D2H");
-        cuda_check(cudaStreamSynchronize(s), "params");
-        out.insert(out.end(), w.begin(), w.end());
-        out.insert(out.end(), b.begin(), b.end());
-    }
+    out.resize(kSeedParams);
+    cuda_check(cudaMemcpyAsync(out.data(), P.p, kSeedParams * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
+    cuda_check(cudaStreamSynchronize(s), "params");
 }
 
 void SeedModel::set_params(const float *p, size_t n) {
     if ((int)n != params()) throw Error(ERR_FORMAT, "seed parameter count mismatch");
     if (!s) cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     if (spec[0].cin == 0) set_tile(kSeedS, kSeedHalo);
-    size_t o = 0;
-    for (int i = 0; i < kSeedConvs; i++) {
-        const int nw = kCout[i] * 9 * kCin[i];
-        set_layer(i, p + o, p + o + nw);
-        o += nw + kCout[i];
+    P.upload(p, n, s);
+    for (auto *buf : {&mP, &vP, &acc, &G}) {
+        buf->alloc(n);
+        cuda_check(cudaMemsetAsync(buf->p, 0, n * sizeof(float), s), "memset");
     }
+    W.alloc(n);
+    WT.alloc(n);
+    launch_seed_weights(P.p, W.p, WT.p, s);
+    cuda_check(cudaStreamSynchronize(s), "seed weights");
     adam_t = 0;
 }
 
@@ -161,7 +127,7 @@ void SeedModel::forward(int T) {
     const __nv_bfloat16 *in = x0.p;
     for (int i = 0; i < kSeedConvs; i++) {
         const bool last = i == kSeedConvs - 1;
-        launch_conv_fwd(spec[i], T, in, W[i].p, bias[i].p, last ? y16.p : act[i].p, last ? y32.p : nullptr, err.p, s);
+        launch_conv_fwd(spec[i], T, in, W.p + seed_at(i), P.p + seed_bias_at(i), last ? y16.p : act[i].p, last ? y32.p : nullptr, err.p, s);
         if (!last) in = act[i].p;
     }
 }
@@ -177,7 +143,7 @@ void SeedModel::time_forward(int T, int reps, double *layer_ms, double *layer_fl
         cuda_check(cudaEventRecord(ev[0], s), "event");
         for (int i = 0; i < kSeedConvs; i++) {
             const bool last = i == kSeedConvs - 1;
-            launch_conv_fwd(spec[i], T, in, W[i].p, bias[i].p, last ? y16.p : act[i].p, last ? y32.p : nullptr,
+            launch_conv_fwd(spec[i], T, in, W.p + seed_at(i), P.p + seed_bias_at(i), last ? y16.p : act[i].p, last ? y32.p : nullptr,
                             err.p, s);
             if (!last) in = act[i].p;
             cuda_check(cudaEventRecord(ev[i + 1], s), "event");
@@ -199,20 +165,15 @@ void SeedModel::time_forward(int T, int reps, double *layer_ms, double *layer_fl
 
 double SeedModel::backward(int T, double *mae) {
     cuda_check(cudaMemsetAsync(sums.p, 0, 2 * sizeof(double), s), "memset");
-    launch_seed_loss(T, S, halo, y32.p, tgt32.p, grad[5].p, sums.p, s);
-    for (int i = 0; i < kSeedConvs; i++) {
-        const int n = kCout[i] * 9 * kCin[i];
-        cuda_check(cudaMemsetAsync(dWT[i].p, 0, n * sizeof(float), s), "memset");
-        cuda_check(cudaMemsetAsync(db[i].p, 0, kCout[i] * sizeof(float), s), "memset");
-    }
+    cuda_check(cudaMemsetAsync(acc.p, 0, kSeedParams * sizeof(float), s), "memset");
+    launch_seed_loss(T, S, halo, y32.p, tgt32.p, grad[5].p, sums.p, acc.p + seed_bias_at(kSeedConvs - 1), s);
     for (int i = kSeedConvs - 1; i >= 0; i--) {
         const __nv_bfloat16 *X = i == 0 ? x0.p : act[i - 1].p;
-        launch_conv_wgrad(spec[i], T, X, grad[i].p, dWT[i].p, err.p, s);
-        if (i == kSeedConvs - 1) launch_bias_grad(spec[i], T, grad[i].p, db[i].p, s);
+        launch_conv_wgrad(spec[i], T, X, grad[i].p, acc.p + seed_at(i), err.p, s);
         if (i > 0)
-            launch_conv_dgrad(spec[i], T, grad[i].p, WT[i].p, act[i - 1].p, grad[i - 1].p, db[i - 1].p, err.p, s);
+            launch_conv_dgrad(spec[i], T, grad[i].p, WT.p + seed_at(i), act[i - 1].p, grad[i - 1].p,
+                              acc.p + seed_bias_at(i - 1), err.p, s);
     }
-    for (int i = 0; i < kSeedConvs; i++) launch_seed_grad_layout(kCin[i], kCout[i], dWT[i].p, dW[i].p, s);
     double h[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(h, sums.p, sizeof h, cudaMemcpyDeviceToHost, s), "D2H");
     check("backward");
@@ -223,25 +184,14 @@ double SeedModel::backward(int T, double *mae) {
 
 void SeedModel::adam(float lr) {
     adam_t++;
-    for (int i = 0; i < kSeedConvs; i++) {
-        const int n = kCout[i] * 9 * kCin[i];
-        launch_adam(n, Wm[i].p, dW[i].p, mW[i].p, vW[i].p, lr, 0.9f, 0.999f, 1e-8f, adam_t, s);
-        launch_adam(kCout[i], bias[i].p, db[i].p, mb[i].p, vb[i].p, lr, 0.9f, 0.999f, 1e-8f, adam_t, s);
-        launch_seed_weights(kCin[i], kCout[i], Wm[i].p, W[i].p, WT[i].p, s);
-    }
+    launch_adam(P.p, mP.p, vP.p, acc.p, W.p, WT.p, lr, 0.9f, 0.999f, 1e-8f, adam_t, s);
 }
 
 void SeedModel::grads(std::vector<float> &out) {
-    out.clear();
-    for (int i = 0; i < kSeedConvs; i++) {
-        const int n = kCout[i] * 9 * kCin[i];
-        std::vector<float> w(n), b(kCout[i]);
-        cuda_check(cudaMemcpyAsync(w.data(), dW[i].p, n * 4, cudaMemcpyDeviceToHost, s), "D2H");
-        cuda_check(cudaMemcpyAsync(b.data(), db[i].p, kCout[i] * 4, cudaMemcpyDeviceToHost, s), "D2H");
-        cuda_check(cudaStreamSynchronize(s), "grads");
-        out.insert(out.end(), w.begin(), w.end());
-        out.insert(out.end(), b.begin(), b.end());
-    }
+    out.resize(kSeedParams);
+    launch_seed_grad_layout(acc.p, G.p, s);
+    cuda_check(cudaMemcpyAsync(out.data(), G.p, kSeedParams * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
+    cuda_check(cudaStreamSynchronize(s), "grads");
 }
 
 // ---------------------------------------------------------------- data
@@ -287,8 +237,7 @@ double SeedModel::train(int steps, int T, float lr, uint64_t seed, std::vector<d
             tr[t].y0 = m.Y > inner ? (int)(splitmix(r) % (uint64_t)(m.Y - inner + 1)) : 0;
         }
         cuda_check(cudaMemcpyAsync(tiles.p, tr.data(), T * sizeof(TileRef), cudaMemcpyHostToDevice, s), "H2D");
-        launch_gather_tiles(T, S, halo, tiles.p, fpool.p, x0.p, nullptr, s);
-        launch_gather_tiles(T, S, halo, tiles.p, tpool.p, nullptr, tgt32.p, s);
+        launch_gather_tiles(T, S, halo, tiles.p, fpool.p, x0.p, tpool.p, tgt32.p, s);
         forward(T);
         last = backward(T, nullptr);
         adam(lr);
@@ -310,7 +259,7 @@ void SeedModel::predict(int X, int Y, const __nv_bfloat16 *feat_dev, float *pred
     for (int t0 = 0; t0 < nt; t0 += T) {
         const int n = std::min(T, nt - t0);
         cuda_check(cudaMemcpyAsync(tiles.p, tr.data() + t0, n * sizeof(TileRef), cudaMemcpyHostToDevice, s), "H2D");
-        launch_gather_tiles(n, S, halo, tiles.p, feat_dev, x0.p, nullptr, s);
+        launch_gather_tiles(n, S, halo, tiles.p, feat_dev, x0.p, nullptr, nullptr, s);
         forward(n);
         launch_scatter_prediction(n, S, halo, tiles.p, y32.p, pred_dev, s);
     }

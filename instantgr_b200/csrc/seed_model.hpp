@@ -9,11 +9,11 @@ struct SeedModel {
     int S = 0, halo = 0;
     ConvSpec spec[kSeedConvs] = {};
     cudaStream_t s = nullptr;
-    // parameters: f32 master weights [cout][9][cin], biases, Adam moments,
-    // gradients, and the BF16 working copies W and WT ([cin][9][cout])
-    DevBuf<float> Wm[kSeedConvs], bias[kSeedConvs], mW[kSeedConvs], vW[kSeedConvs], dW[kSeedConvs],
-        dWT[kSeedConvs], mb[kSeedConvs], vb[kSeedConvs], db[kSeedConvs];
-    DevBuf<__nv_bfloat16> W[kSeedConvs], WT[kSeedConvs];
+    // all parameters end to end (seed_at): f32 master copy, Adam moments,
+    // gradient sums as the convolutions leave them, gradients in parameter
+    // order, and the BF16 working weights W and WT ([cin][9][cout])
+    DevBuf<float> P, mP, vP, acc, G;
+    DevBuf<__nv_bfloat16> W, WT;
     int adam_t = 0;
     // activations of up to Tcap tiles: input, outputs of c1..c5, gradients of
     // the pre-activations of c1..c6, output (bf16 and f32) and target
@@ -31,7 +31,7 @@ struct SeedModel {
     ~SeedModel();
     void set_tile(int S, int halo);   // tile size with halo (even), halo
     void init(uint64_t seed);         // He-normal weights, zero biases
-    int params() const;               // weights then bias of each layer
+    int params() const { return kSeedParams; }  // weights then bias of each layer
     void get_params(std::vector<float> &out);
     void set_params(const float *p, size_t n);
     void ensure(int T);
@@ -52,9 +52,6 @@ struct SeedModel {
     // [3] MAE of predicting each layer's mean demand over the map
     void evaluate(int map, double *out);
     void check(const char *what);
-
-   private:
-    void set_layer(int i, const float *w, const float *b);
 };
 
 // 16-channel features of a design, [X][Y][16]: pins, RUDY-H, RUDY-V, blocked
