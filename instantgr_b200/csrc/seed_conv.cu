@@ -13,7 +13,7 @@
 // the tile's even and odd columns lie apart and the row groups skip a row.
 //
 // A block runs over tiles with three roles: four warps copy source tiles
-// (cp.async, three in flight), one thread issues a tile's MMAs, four warps write
+// (cp.async, three in flight), one thread issues a tile's MMAs, eight warps write
 // the previous tile's results from TMEM (two stages).  The weights stay in
 // shared memory.  What bounds it: the MMAs read their operands from shared
 // memory, 6 KB for 128 x 64 x 16, so N = 64 cannot pass a third of the tensor
@@ -21,8 +21,10 @@
 // gradients also read the mask and keep the sums of the bias gradients.
 // Gathering each tap's operands anew through registers, as the kernel before it
 // did, moved nine times the tile.  16 tiles of 288 x 288: forward pass 2.03 ->
-// 0.37 ms (135 GFLOP, 365 TFLOP/s), input gradients with the bias gradients
-// 2.10 + 0.56 -> 0.47 ms.
+// 0.37 ms (135 GFLOP, 350 TFLOP/s by events around each convolution), input
+// gradients with the bias gradients 2.10 + 0.56 -> 0.40 ms.  Of the 49 us of a
+// 64-channel layer 18 go to the MMAs, 6 to the copies, 5 to the stores and 20 to
+// the launch and the hand-over between the roles (measured by leaving each out).
 //
 // The K order of every output is tap by tap and 16 channels at a time.  Every
 // wait is bounded (ERR_TIMEOUT in the error word) and the TMEM columns are freed
@@ -51,6 +53,7 @@ template <Kind K, int CIN, int N>
 struct Geo {
     static constexpr bool fine = K == kUp2 || K == kStride2T;   // output at twice the tile grid's resolution
     static constexpr bool half = K == kStride2 || K == kUp2T;   // source at twice the tile grid's resolution
+    static_assert(K != kStride2 && K != kUp2T || N >= 32, "a group's columns");
     static constexpr int gemms = K == kSame ? 2 : fine ? 4 : 1;  // 128-row GEMMs of a tile
     static constexpr int rows = 16, cols = K == kSame ? 16 : 8;  // tile, in the tile grid's pixels
     // source pixels of a tile, the pitch of their rows and their places in a plane
@@ -87,13 +90,14 @@ struct ConvArgs {
     int probe;
 };
 
-constexpr int kConvThreads = 288;
+constexpr int kConvThreads = 416;  // warps 0-7 results, 8-11 copies, 12 MMAs
+constexpr int kWgradThreads = 288;
 
 template <Kind K, int CIN, int N, bool GRAD, int MINB>
 __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs p) {
     using G = Geo<K, CIN, N>;
     extern __shared__ __align__(128) uint8_t sm[];
-    __shared__ __align__(8) uint64_t full[G::bufs], empty[G::bufs], tfull[2], tempty[2];
+    __shared__ __align__(8) uint64_t full[G::bufs], empty[G::bufs], tfull[2], tempty[2], weights;
     __shared__ uint32_t tbase;
     __shared__ volatile int quit;
     __shared__ __align__(16) float sbias[N];
@@ -108,21 +112,13 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
         }
         for (int i = 0; i < 2; i++) {
             umma::mbar_init(&tfull[i]);
-            umma::mbar_init(&tempty[i], 128);
+            umma::mbar_init(&tempty[i], 256);
         }
+        umma::mbar_init(&weights, 256);
         umma::mbar_init_fence();
-    }
-    // weights: a sub-tile of N x 16 per tap and 16 channels
-    for (int q = tid; q < 9 * G::chunks * N; q += kConvThreads) {
-        const int k8 = q % (9 * G::chunks), n = q / (9 * G::chunks);
-        umma::copy16(umma::smem_u32(sB) + (k8 >> 1) * (N * 32) + (n >> 3) * 256 + (k8 & 1) * 128 + (n & 7) * 16,
-                     p.w + (size_t)n * 9 * CIN + k8 * 8, true);
     }
     if constexpr (!GRAD)
         for (int n = tid; n < N; n += kConvThreads) sbias[n] = p.bias[n];
-    umma::copy_commit();
-    umma::copy_wait<0>();
-    umma::fence_async_smem();
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
@@ -141,9 +137,9 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
         y0 = r / p.tx * G::rows;
         x0 = (r - r / p.tx * p.tx) * G::cols;
     };
-    if (warp >= 4 && warp < 8) {
+    if (warp >= 8 && warp < 12) {
         // ---- copies of the source tiles
-        const int pt = tid - 128;
+        const int pt = tid - 256;
         for (int it = 0; it < mine; it++) {
             const int b = it % G::bufs;
             if (it >= G::bufs) ok = umma::mbar_wait(&empty[b], (it / G::bufs - 1) & 1, p.wait_ns, &quit);
@@ -171,12 +167,13 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
         umma::copy_wait<0>();
         umma::fence_async_smem();
         if (ok && mine > 0) umma::mbar_arrive(&full[(mine - 1) % G::bufs]);
-    } else if (tid == 256) {
+    } else if (tid == 384) {
         // ---- MMAs of a tile, per GEMM tap by tap and 16 channels at a time
         constexpr uint32_t idesc = umma::idesc_bf16(128, N);
         const uint64_t db = umma::smem_desc(umma::smem_u32(sB));
         int issued = 0;
-        for (int it = 0; it < mine; it++) {
+        if (mine > 0) ok = umma::mbar_wait(&weights, 0, p.wait_ns, &quit);
+        for (int it = 0; it < mine && ok; it++) {
             const int b = it % G::bufs, s = it & 1;
             ok = umma::mbar_wait(&full[b], (it / G::bufs) & 1, p.wait_ns, &quit);
             if (ok && it >= 2) ok = umma::mbar_wait(&tempty[s], ((it >> 1) - 1) & 1, p.wait_ns, &quit);
@@ -225,32 +222,47 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
         }
         // every issued MMA has completed once the last commit has
         if (issued > 0 && !umma::mbar_wait(&tfull[(issued - 1) & 1], ((issued - 1) >> 1) & 1, kDrainNs)) ok = false;
-    } else if (warp < 4) {
-        // ---- results: thread = row of the GEMMs = pixel
-        const int r = tid >> 3, c = tid & 7;
-        float sum[GRAD ? N : 1];
+    } else if (warp < 8) {
+        // ---- weights first: a sub-tile of N x 16 per tap and 16 channels
+        for (int q = tid; q < 9 * G::chunks * N; q += 256) {
+            const int k8 = q % (9 * G::chunks), n = q / (9 * G::chunks);
+            umma::copy16(umma::smem_u32(sB) + (k8 >> 1) * (N * 32) + (n >> 3) * 256 + (k8 & 1) * 128 + (n & 7) * 16,
+                         p.w + (size_t)n * 9 * CIN + k8 * 8, true);
+        }
+        umma::copy_commit();
+        umma::copy_wait<0>();
+        umma::fence_async_smem();
+        umma::mbar_arrive(&weights);
+        // ---- results: thread = row of the GEMMs = pixel; the two groups of four warps
+        //      share a tile's GEMMs, or the columns of a single one
+        constexpr int kCols = G::gemms == 1 ? N / 2 : N;  // columns of a group
+        constexpr int kBatch = kCols < 32 ? kCols : 32;   // columns in flight
+        const int group = warp >> 2, r = (tid & 127) >> 3, c = tid & 7;
+        const int col0 = G::gemms == 1 ? group * kCols : 0;
+        float sum[GRAD ? kCols : 1];
         if constexpr (GRAD)
-            for (int n = 0; n < N; n++) sum[n] = 0.f;
+            for (int n = 0; n < kCols; n++) sum[n] = 0.f;
         for (int it = 0; it < mine; it++) {
             const int s = it & 1;
             int img, y0, x0;
             tile_at(it, img, y0, x0);
             bool in = false;
             size_t at = 0;
-            uint4 m[GRAD ? N / 8 : 1];  // a GEMM's masks, on their way while its MMAs run
+            uint4 m[GRAD ? kCols / 8 : 1];  // a GEMM's masks, on their way while its MMAs run
             auto pixel = [&](int j) {
                 const int y = G::fine ? 2 * (y0 + r) + (j >> 1) : y0 + r;
                 const int x = G::fine ? 2 * (x0 + c) + (j & 1) : x0 + c + 8 * j;
                 in = y < p.oh && x < p.ow;
-                at = in ? (((size_t)img * p.oh + y) * p.ow + x) * N : 0;
+                at = in ? (((size_t)img * p.oh + y) * p.ow + x) * N + col0 : 0;
                 if constexpr (GRAD) {
                     if (p.mask) {
 #pragma unroll
-                        for (int i = 0; i < N / 8; i++) m[i] = reinterpret_cast<const uint4 *>(p.mask + at)[i];
+                        for (int i = 0; i < kCols / 8; i++) m[i] = reinterpret_cast<const uint4 *>(p.mask + at)[i];
                     }
                 }
             };
-            pixel(0);
+            const int j0 = G::gemms == 1 ? 0 : group;
+            pixel(j0);
             ok = umma::mbar_wait(&tfull[s], (it >> 1) & 1, p.wait_ns, &quit);
             if (!__all_sync(0xffffffffu, ok)) {
                 ok = false;
@@ -258,55 +270,64 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
             }
             umma::fence_after();
 #pragma unroll
-            for (int j = 0; j < G::gemms; j++) {
-                if (j > 0) pixel(j);
+            for (int jj = 0; jj < (G::gemms + 1) / 2; jj++) {
+                const int j = j0 + 2 * jj;
+                if (jj > 0) pixel(j);
 #pragma unroll
-                for (int n0 = 0; n0 < N; n0 += 16) {
-                    uint32_t v[16];
-                    umma::tmem_ld(tmem + ((uint32_t)(warp * 32) << 16) + s * G::stage + j * N + n0, v);
+                for (int b0 = 0; b0 < kCols; b0 += kBatch) {
+                    uint32_t v[kBatch / 16][16];
+#pragma unroll
+                    for (int k = 0; k < kBatch / 16; k++)
+                        umma::tmem_ld(tmem + ((uint32_t)((warp & 3) * 32) << 16) + s * G::stage + j * N + col0 + b0 +
+                                          16 * k, v[k]);
                     umma::tmem_wait();
-                    uint32_t o[8];
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        float a = __uint_as_float(v[2 * i]), b = __uint_as_float(v[2 * i + 1]);
-                        if constexpr (GRAD) {
-                            if (p.mask) {
-                                const uint4 q = m[n0 / 8 + i / 4];
-                                const uint32_t w = i % 4 == 0 ? q.x : i % 4 == 1 ? q.y : i % 4 == 2 ? q.z : q.w;
-                                a = __uint_as_float(w << 16) > 0.f ? a : 0.f;
-                                b = __uint_as_float(w & 0xffff0000u) > 0.f ? b : 0.f;
+                    for (int k = 0; k < kBatch / 16; k++) {
+                        const int n0 = b0 + 16 * k;
+                        uint32_t o[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            float a = __uint_as_float(v[k][2 * i]), b = __uint_as_float(v[k][2 * i + 1]);
+                            if constexpr (GRAD) {
+                                if (p.mask) {
+                                    const uint4 q = m[n0 / 8 + i / 4];
+                                    const uint32_t w = i % 4 == 0 ? q.x : i % 4 == 1 ? q.y : i % 4 == 2 ? q.z : q.w;
+                                    a = __uint_as_float(w << 16) > 0.f ? a : 0.f;
+                                    b = __uint_as_float(w & 0xffff0000u) > 0.f ? b : 0.f;
+                                }
+                            } else {
+                                const float2 bb = *reinterpret_cast<const float2 *>(&sbias[col0 + n0 + 2 * i]);
+                                a += bb.x;
+                                b += bb.y;
+                                if (p.relu) {
+                                    a = fmaxf(a, 0.f);
+                                    b = fmaxf(b, 0.f);
+                                }
+                                v[k][2 * i] = __float_as_uint(a);
+                                v[k][2 * i + 1] = __float_as_uint(b);
                             }
-                        } else {
-                            a += sbias[n0 + 2 * i];
-                            b += sbias[n0 + 2 * i + 1];
-                            if (p.relu) {
-                                a = fmaxf(a, 0.f);
-                                b = fmaxf(b, 0.f);
+                            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+                            o[i] = *reinterpret_cast<const uint32_t *>(&h);
+                            if constexpr (GRAD) {
+                                if (in) {
+                                    sum[n0 + 2 * i] += __bfloat162float(h.x);
+                                    sum[n0 + 2 * i + 1] += __bfloat162float(h.y);
+                                }
                             }
-                            v[2 * i] = __float_as_uint(a);
-                            v[2 * i + 1] = __float_as_uint(b);
                         }
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-                        o[i] = *reinterpret_cast<const uint32_t *>(&h);
-                        if constexpr (GRAD) {
-                            if (in) {
-                                sum[n0 + 2 * i] += __bfloat162float(h.x);
-                                sum[n0 + 2 * i + 1] += __bfloat162float(h.y);
-                            }
+                        if (in) {
+                            umma::store32(p.out + at + n0, o);
+                            if constexpr (!GRAD)
+                                if (p.out32) {
+                                    uint32_t h[8];
+#pragma unroll
+                                    for (int i = 0; i < 8; i++) h[i] = v[k][i];
+                                    umma::store32(p.out32 + at + n0, h);
+#pragma unroll
+                                    for (int i = 0; i < 8; i++) h[i] = v[k][8 + i];
+                                    umma::store32(p.out32 + at + n0 + 8, h);
+                                }
                         }
-                    }
-                    if (in) {
-                        umma::store32(p.out + at + n0, o);
-                        if constexpr (!GRAD)
-                            if (p.out32) {
-                                uint32_t h[8];
-#pragma unroll
-                                for (int i = 0; i < 8; i++) h[i] = v[i];
-                                umma::store32(p.out32 + at + n0, h);
-#pragma unroll
-                                for (int i = 0; i < 8; i++) h[i] = v[8 + i];
-                                umma::store32(p.out32 + at + n0 + 8, h);
-                            }
                     }
                 }
             }
@@ -316,18 +337,19 @@ __global__ void __launch_bounds__(kConvThreads, MINB) conv_kernel(const ConvArgs
         if constexpr (GRAD) {
             if (p.db && ok && mine > 0) {
                 // sums over the lanes: half of the channels change hands at each step,
-                // until lane l has channels l N / 32 ..
+                // until lane l has channels l kCols / 32 ..
 #pragma unroll
-                for (int o = 16, half = N / 2; o > 0; o >>= 1, half /= 2) {
+                for (int st = 0; st < 5; st++) {
+                    const int o = 16 >> st, half = kCols >> (st + 1);
                     const bool up = lane & o;
 #pragma unroll
-                    for (int n = 0; n < half; n++) {
+                    for (int n = 0; n < (kCols >> (st + 1)); n++) {
                         const float give = up ? sum[n] : sum[n + half];
                         sum[n] = (up ? sum[n + half] : sum[n]) + __shfl_xor_sync(0xffffffffu, give, o);
                     }
                 }
 #pragma unroll
-                for (int n = 0; n < N / 32; n++) atomicAdd(p.db + lane * (N / 32) + n, sum[n]);
+                for (int n = 0; n < kCols / 32; n++) atomicAdd(p.db + col0 + lane * (kCols / 32) + n, sum[n]);
             }
         }
     }
@@ -420,7 +442,7 @@ __device__ __forceinline__ void add4(float *p, float a, float b, float c, float 
 }
 
 template <WKind K, bool AX, int CA, int CB, int CBALL>
-__global__ void __launch_bounds__(kConvThreads, 1) wgrad_kernel(const WgradArgs p) {
+__global__ void __launch_bounds__(kWgradThreads, 1) wgrad_kernel(const WgradArgs p) {
     using G = WGeo<K, AX, CA, CB, CBALL>;
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ __align__(8) uint64_t full[G::bufs], empty[G::bufs], done;
@@ -610,13 +632,13 @@ void launch_wgrad(WgradArgs a, int T, int halves, cudaStream_t s) {
     constexpr int smem = G::smem > floor_bytes ? G::smem : floor_bytes;
     static_assert(smem <= 227 * 1024, "a block's shared memory");
     const auto kernel = wgrad_kernel<K, AX, CA, CB, CBALL>;
-    const KernelShape ks = kernel_setup((const void *)kernel, kConvThreads, smem);
+    const KernelShape ks = kernel_setup((const void *)kernel, kWgradThreads, smem);
     a.ty = (a.ah + G::rows - 1) / G::rows;
     a.tx = (a.aw + 15) / 16;
     a.tiles = T * a.ty * a.tx;
     a.wait_ns = (unsigned long long)test_hooks().wait_ns.load();
     a.probe = test_hooks().mbar_probe.load();
-    kernel<<<dim3(std::min(a.tiles, ks.sms / halves), halves), kConvThreads, smem, s>>>(a);
+    kernel<<<dim3(std::min(a.tiles, ks.sms / halves), halves), kWgradThreads, smem, s>>>(a);
 }
 
 [[noreturn]] void no_kernel(const ConvSpec &c) {
@@ -632,7 +654,7 @@ void launch_conv_fwd(const ConvSpec &c, int T, const __nv_bfloat16 *X, const __n
     a.src = X; a.w = W; a.sh = c.hin; a.sw = c.win; a.oh = c.hout; a.ow = c.wout;
     a.relu = c.relu; a.bias = bias; a.out = Y; a.out32 = Y32; a.err = err;
     const int key = c.mode * 10000 + c.cin * 100 + c.cout;
-    if (key == 1632) launch<kSame, 16, 32, false, 3>(a, T, c.hout, c.wout, s);
+    if (key == 1632) launch<kSame, 16, 32, false, 2>(a, T, c.hout, c.wout, s);
     else if (key == 6464) launch<kSame, 64, 64, false, 1>(a, T, c.hout, c.wout, s);
     else if (key == 3216) launch<kSame, 32, 16, false, 2>(a, T, c.hout, c.wout, s);
     else if (key == 13264) launch<kStride2, 32, 64, false, 1>(a, T, c.hout, c.wout, s);
@@ -647,8 +669,8 @@ void launch_conv_dgrad(const ConvSpec &c, int T, const __nv_bfloat16 *dY, const 
     a.mask = Aprev; a.out = dXpre; a.db = db; a.err = err;
     const int key = c.mode * 10000 + c.cin * 100 + c.cout;
     if (key == 6464) launch<kSame, 64, 64, true, 1>(a, T, c.hin, c.win, s);
-    else if (key == 3216) launch<kSame, 16, 32, true, 2>(a, T, c.hin, c.win, s);
-    else if (key == 13264) launch<kStride2T, 64, 32, true, 2>(a, T, c.hout, c.wout, s);
+    else if (key == 3216) launch<kSame, 16, 32, true, 1>(a, T, c.hin, c.win, s);
+    else if (key == 13264) launch<kStride2T, 64, 32, true, 1>(a, T, c.hout, c.wout, s);
     else if (key == 26432) launch<kUp2T, 32, 64, true, 1>(a, T, c.hin, c.win, s);
     else no_kernel(c);
 }
