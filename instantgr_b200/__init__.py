@@ -579,7 +579,7 @@ class Seed:
 
     def predict(self, features) -> np.ndarray:
         f = np.ascontiguousarray(features, dtype=np.float32)
-        out = np.zeros_like(f)
+        out = np.empty_like(f)  # written in full
         self._c(lib().igr_seed_predict(self.h, f.shape[0], f.shape[1], f.reshape(-1), out.reshape(-1)))
         return out
 

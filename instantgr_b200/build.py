@@ -25,7 +25,7 @@ CUDA_INC = "/usr/local/cuda/include"
 
 CU_SOURCES = ["cost.cu", "commit.cu", "ripup.cu", "pattern.cu", "pattern_static.cu", "color.cu", "dag.cu", "plan.cu",
               "seed_conv.cu", "seed_nn.cu", "seed_feat.cu", "shapes.cu", "eval.cu", "records.cu", "dagbuild.cu", "launch.cu"]
-CPP_SOURCES = ["design_io.cpp", "pins.cpp", "netbuild.cpp", "gen.cpp", "dag_build.cpp", "dag_device.cpp", "router.cpp",
+CPP_SOURCES = ["design_io.cpp", "pins.cpp", "netbuild.cpp", "gen.cpp", "dag_build.cpp", "dag_device.cpp", "host_copy.cpp", "router.cpp",
                "capi.cpp", "seed_model.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # --fmad=false: the only multiply-add the reference contracts is written as fma() explicitly

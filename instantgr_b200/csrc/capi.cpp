@@ -245,8 +245,7 @@ int igr_router_demand(igr_router *h, float *out) {
         DevBuf<float> t;
         t.alloc(r.go.g.N);
         launch_from_track_layout_f(r.go.g, r.go.demand.p, t.p, r.s);
-        cuda_check(cudaMemcpyAsync(out, t.p, r.go.g.N * sizeof(float), cudaMemcpyDeviceToHost, r.s), "D2H");
-        cuda_check(cudaStreamSynchronize(r.s), "sync");
+        copy_to_host(out, t.p, r.go.g.N * sizeof(float), r.s);
     });
 }
 
@@ -989,12 +988,6 @@ int igr_router_seed_stats(igr_router *h, double *out, int n) {
         return guard(&(m)->err, [&] { __VA_ARGS__; });                          \
     } while (0)
 
-static std::vector<__nv_bfloat16> to_bf16(const float *p, size_t n) {
-    std::vector<__nv_bfloat16> v(n);
-    for (size_t i = 0; i < n; i++) v[i] = __float2bfloat16(p[i]);
-    return v;
-}
-
 int igr_seed_create(uint64_t init_seed, igr_seed **out) {
     if (!out) return fail(nullptr, IGR_ERR_INVALID, "null argument");
     *out = nullptr;
@@ -1067,7 +1060,9 @@ int igr_seed_add_map(igr_seed *m, int X, int Y, const float *feat, const float *
     SEED_GUARD(m, {
         if (X < 1 || Y < 1 || !feat || !target) throw Error(ERR_INVALID, "bad map");
         const size_t n = (size_t)X * Y * 16;
-        const auto f = to_bf16(feat, n), t = to_bf16(target, n);
+        std::vector<__nv_bfloat16> f(n), t(n);
+        convert_to_bf16(feat, n, f.data());
+        convert_to_bf16(target, n, t.data());
         const int id = m->m.add_map(X, Y, f.data(), t.data());
         if (map_id) *map_id = id;
     });
@@ -1126,15 +1121,14 @@ int igr_seed_predict(igr_seed *m, int X, int Y, const float *feat, float *pred) 
     SEED_GUARD(m, {
         if (X < 1 || Y < 1 || !feat || !pred) throw Error(ERR_INVALID, "bad map");
         const size_t n = (size_t)X * Y * 16;
-        const auto f = to_bf16(feat, n);
         DevBuf<__nv_bfloat16> fd;
         DevBuf<float> pd;
-        fd.upload(f.data(), n, m->m.s);
+        fd.alloc(n);
+        copy_to_device_bf16(fd.p, feat, n, m->m.s);
         pd.alloc(n);
         cuda_check(cudaMemsetAsync(pd.p, 0, n * 4, m->m.s), "memset");
         m->m.predict(X, Y, fd.p, pd.p);
-        cuda_check(cudaMemcpyAsync(pred, pd.p, n * 4, cudaMemcpyDeviceToHost, m->m.s), "D2H");
-        cuda_check(cudaStreamSynchronize(m->m.s), "sync");
+        copy_to_host(pred, pd.p, n * 4, m->m.s);
     });
 }
 
@@ -1144,9 +1138,8 @@ int igr_seed_grad(igr_seed *m, int T, const float *x, const float *target, doubl
         auto &M = m->m;
         M.ensure(T);
         const size_t n = (size_t)T * M.S * M.S * 16;
-        const auto xb = to_bf16(x, n);
-        cuda_check(cudaMemcpyAsync(M.x0.p, xb.data(), n * 2, cudaMemcpyHostToDevice, M.s), "H2D");
-        cuda_check(cudaMemcpyAsync(M.tgt32.p, target, n * 4, cudaMemcpyHostToDevice, M.s), "H2D");
+        copy_to_device_bf16(M.x0.p, x, n, M.s);
+        copy_to_device(M.tgt32.p, target, n * 4, M.s);
         M.forward(T);
         const double l = M.backward(T, nullptr);
         if (loss) *loss = l;

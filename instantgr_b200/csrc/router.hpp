@@ -35,6 +35,16 @@ void pinned_free(void *p, size_t bytes);
 // true when the cache holds a page-locked block for `bytes`
 bool pinned_cached(size_t bytes);
 
+// Copies to and from the caller's pageable memory by several host threads
+// through page-locked chunks (host_copy.cpp), after the work queued on `s`.
+// copy_to_host returns when dst is complete; the others when src may be reused
+// (the last one rounds to BF16 on the way).
+void copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s);
+void copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t s);
+void copy_to_device_bf16(__nv_bfloat16 *dst, const float *src, size_t n, cudaStream_t s);
+// float -> BF16 as __float2bfloat16 rounds
+void convert_to_bf16(const float *src, size_t n, __nv_bfloat16 *out);
+
 template <typename T>
 struct PinnedBuf {
     T *p = nullptr;
