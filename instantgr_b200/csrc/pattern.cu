@@ -106,15 +106,6 @@ __device__ __forceinline__ void count_vias(const GridDev &g, int *vcnt, const in
     }
 }
 
-// v / d for v < 2^31 with rcp = floor((2^32 - 1) / d): the product's high word
-// is the quotient or one below it.
-__device__ __forceinline__ unsigned div_by(unsigned v, unsigned d, unsigned rcp, unsigned &rem) {
-    unsigned q = __umulhi(v, rcp);
-    rem = v - q * d;
-    if (rem >= d) { q++; rem -= d; }
-    return q;
-}
-
 // A node's position in one word: layer in bits 28-31, x in 14-27, y in 0-13
 // (a grid side is at most kMaxTrackCells < 2^14).
 struct PosDecoder {

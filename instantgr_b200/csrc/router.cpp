@@ -1842,19 +1842,22 @@ void Router::evaluate(double *out, double *layer_loss) {
     const int64_t XY = (int64_t)X * Y;
     EvalDev e;
     e.n = N; e.L = L; e.X = X; e.Y = Y; e.DIR = go.g.DIR;
-    ev_sel_off.upload(d.sel_off, s); ev_sel.upload(d.sel, s);
-    ev_extra_off.upload(d.extra_off, s); ev_extra.upload(d.extra, s);
-    ev_sub_off.upload(ns.sub_off, s);
-    ev_route_off.upload(route_off, s);
-    e.sel_off = ev_sel_off.p; e.sel = ev_sel.p; e.extra_off = ev_extra_off.p; e.extra = ev_extra.p;
-    e.sub_off = ev_sub_off.p; e.route_off = ev_route_off.p; e.routes = routes.p;
-    e.cap = go.g.cap; e.xlen = go.g.xlen; e.ylen = go.g.ylen; e.err = go.g.err;
-    if (!d.cap_d.empty()) {  // capacities that are not floats: the exact values, in the track layout
-        ev_capd_ref.upload(d.cap_d.data() + XY, (size_t)L * XY, s);
-        ev_capd.alloc((size_t)L * XY);
-        launch_to_track_layout_d(go.g, ev_capd_ref.p, ev_capd.p, s);
-        e.cap_d = ev_capd.p;
+    // the design's pins do not change between runs; the record offsets are on the device
+    if (!ev_ready) {
+        ev_sel_off.upload(d.sel_off, s); ev_sel.upload(d.sel, s);
+        ev_extra_off.upload(d.extra_off, s); ev_extra.upload(d.extra, s);
+        ev_sub_off.upload(ns.sub_off, s);
+        if (!d.cap_d.empty()) {  // capacities that are not floats: the exact values, in the track layout
+            ev_capd_ref.upload(d.cap_d.data() + XY, (size_t)L * XY, s);
+            ev_capd.alloc((size_t)L * XY);
+            launch_to_track_layout_d(go.g, ev_capd_ref.p, ev_capd.p, s);
+        }
+        ev_ready = true;
     }
+    e.sel_off = ev_sel_off.p; e.sel = ev_sel.p; e.extra_off = ev_extra_off.p; e.extra = ev_extra.p;
+    e.sub_off = ev_sub_off.p; e.route_off = d_route_off.p; e.routes = routes.p;
+    e.cap = go.g.cap; e.xlen = go.g.xlen; e.ylen = go.g.ylen; e.err = go.g.err;
+    if (!d.cap_d.empty()) e.cap_d = ev_capd.p;
     ev_wire.alloc((size_t)go.g.N);
     ev_stacked.alloc((size_t)go.g.N);
     cuda_check(cudaMemsetAsync(ev_wire.p, 0, (size_t)go.g.N * sizeof(int), s), "memset");
@@ -1862,35 +1865,42 @@ void Router::evaluate(double *out, double *layer_loss) {
     ev_cnt.alloc(kEvalLayers + L);
     cuda_check(cudaMemsetAsync(ev_cnt.p, 0, (kEvalLayers + L) * sizeof(unsigned long long), s), "memset");
     e.wire = ev_wire.p; e.stacked = ev_stacked.p; e.total_vias = ev_cnt.p; e.wl = ev_cnt.p + kEvalLayers;
-    // counts per design net, then the via-location offsets and the table sizes
-    ev_vcnt.alloc(std::max(N, 1)); ev_ccnt.alloc(std::max(N, 1));
-    launch_eval_count(e, ev_vcnt.p, ev_ccnt.p, s);
-    std::vector<long long> vc(N), cc(N);
-    if (N) {
-        cuda_check(cudaMemcpyAsync(vc.data(), ev_vcnt.p, N * sizeof(long long), cudaMemcpyDeviceToHost, s), "D2H");
-        cuda_check(cudaMemcpyAsync(cc.data(), ev_ccnt.p, N * sizeof(long long), cudaMemcpyDeviceToHost, s), "D2H");
-    }
-    cuda_check(cudaStreamSynchronize(s), "evaluation counts");
-    std::vector<long long> voff(N + 1, 0);
-    long long ncell = 0;
-    for (int i = 0; i < N; i++) { voff[i + 1] = voff[i] + vc[i]; ncell += cc[i]; }
-    const long long nloc = voff[N];
     if (N > (1 << 28) || X > 65535 || Y > 65535) throw Error(ERR_CAPACITY, "design too large for the evaluation keys");
-    auto table = [](long long n) {
-        unsigned long long t = 64;
-        while (t < 2ull * (unsigned long long)n) t <<= 1;
-        return t;
-    };
-    const unsigned long long wt = table(ncell), vt = table(nloc);
-    ev_voff.upload(voff.data(), N + 1, s);
-    ev_wkeys.alloc(wt); ev_vkeys.alloc(vt); ev_vfirst.alloc(vt);
-    ev_vloc.alloc(std::max<long long>(nloc, 1)); ev_vord.alloc(std::max<long long>(nloc, 1));
-    cuda_check(cudaMemsetAsync(ev_wkeys.p, 0xff, wt * 8, s), "memset");
-    cuda_check(cudaMemsetAsync(ev_vkeys.p, 0xff, vt * 8, s), "memset");
-    cuda_check(cudaMemsetAsync(ev_vfirst.p, 0xff, vt * 4, s), "memset");
-    e.wkeys = ev_wkeys.p; e.wmask = wt - 1; e.vkeys = ev_vkeys.p; e.vmask = vt - 1;
-    e.vfirst = ev_vfirst.p; e.vloc = ev_vloc.p; e.vord = ev_vord.p;
-    launch_eval_marks(e, ev_voff.p, nloc, s);
+    ev_list.alloc((size_t)kEvalClasses * std::max(N, 1));
+    ev_class.alloc(2 * kEvalClasses);
+    cuda_check(cudaMemsetAsync(ev_class.p, 0, 2 * kEvalClasses * sizeof(int), s), "memset");
+    launch_eval_nets(e, ev_list.p, ev_class.p, s);
+    int n_big = 0;
+    cuda_check(cudaMemcpyAsync(&n_big, ev_class.p + kEvalClasses - 1, sizeof n_big, cudaMemcpyDeviceToHost, s), "D2H");
+    cuda_check(cudaStreamSynchronize(s), "evaluation");
+    if (n_big > 0) {  // nets of very many lines: hash sets sized for their cells and via locations
+        const int *big = ev_list.p + (size_t)(kEvalClasses - 1) * N;
+        ev_vcnt.alloc(n_big); ev_ccnt.alloc(n_big);
+        launch_eval_count(e, n_big, big, ev_vcnt.p, ev_ccnt.p, s);
+        std::vector<long long> vc(n_big), cc(n_big);
+        cuda_check(cudaMemcpyAsync(vc.data(), ev_vcnt.p, n_big * sizeof(long long), cudaMemcpyDeviceToHost, s), "D2H");
+        cuda_check(cudaMemcpyAsync(cc.data(), ev_ccnt.p, n_big * sizeof(long long), cudaMemcpyDeviceToHost, s), "D2H");
+        cuda_check(cudaStreamSynchronize(s), "evaluation counts");
+        std::vector<long long> voff(n_big + 1, 0);
+        long long ncell = 0;
+        for (int i = 0; i < n_big; i++) { voff[i + 1] = voff[i] + vc[i]; ncell += cc[i]; }
+        const long long nloc = voff[n_big];
+        auto table = [](long long n) {
+            unsigned long long t = 64;
+            while (t < 2ull * (unsigned long long)n) t <<= 1;
+            return t;
+        };
+        const unsigned long long wt = table(ncell), vt = table(nloc);
+        ev_voff.upload(voff.data(), n_big + 1, s);
+        ev_wkeys.alloc(wt); ev_vkeys.alloc(vt); ev_vfirst.alloc(vt);
+        ev_vloc.alloc(std::max<long long>(nloc, 1)); ev_vord.alloc(std::max<long long>(nloc, 1));
+        cuda_check(cudaMemsetAsync(ev_wkeys.p, 0xff, wt * 8, s), "memset");
+        cuda_check(cudaMemsetAsync(ev_vkeys.p, 0xff, vt * 8, s), "memset");
+        cuda_check(cudaMemsetAsync(ev_vfirst.p, 0xff, vt * 4, s), "memset");
+        e.wkeys = ev_wkeys.p; e.wmask = wt - 1; e.vkeys = ev_vkeys.p; e.vmask = vt - 1;
+        e.vfirst = ev_vfirst.p; e.vloc = ev_vloc.p; e.vord = ev_vord.p;
+        launch_eval_marks(e, n_big, big, ev_voff.p, nloc, s);
+    }
     const int bpl = eval_blocks_per_layer(XY);
     ev_part.alloc((size_t)bpl * L);
     launch_eval_cells(e, bpl, ev_part.p, s);

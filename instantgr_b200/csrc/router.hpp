@@ -346,8 +346,9 @@ struct Router {
     // (run/evaluator.cpp:462-633): out = {wirelength cost, via cost, overflow
     // cost, total}; layer_loss (optional, L entries) = overflow loss per routing layer.
     void evaluate(double *out, double *layer_loss);
-    DevBuf<int64_t> ev_sel_off, ev_extra_off, ev_route_off;
-    DevBuf<int> ev_sel, ev_extra, ev_sub_off, ev_wire, ev_stacked;
+    bool ev_ready = false;  // pins and exact capacities on the device
+    DevBuf<int64_t> ev_sel_off, ev_extra_off;
+    DevBuf<int> ev_sel, ev_extra, ev_sub_off, ev_wire, ev_stacked, ev_list, ev_class;
     DevBuf<long long> ev_vcnt, ev_ccnt, ev_voff;
     DevBuf<unsigned long long> ev_cnt, ev_wkeys, ev_vkeys, ev_vloc;
     DevBuf<unsigned> ev_vfirst, ev_vord;
