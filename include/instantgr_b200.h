@@ -98,8 +98,8 @@ int igr_router_stats(igr_router *r, double *out, int n);
  * refresh}, out[3k] = launches, out[3k+1] = milliseconds, out[3k+2] =
  * algorithmic DRAM bytes (cost refresh: 20 per refreshed cell; fused commit
  * and refresh: 20 per refreshed cell + 12 per committed cell;
- * colouring: 12 per claimed cell, 8 per commit point check, 12 per blocking
- * point check, 8 per release check, 8 per active-list entry scanned; tree
+ * colouring: 12 per claimed cell, 8 per commit or blocking point check, 8 per
+ * cell checked when a net joins, 8 per active-list entry scanned; tree
  * DP: 32 per node, 144 per straight and 360 per bent tree edge). */
 int igr_router_kstats(igr_router *r, double *out, int n);
 /* Phase-1 plan of the last run: routing order, batch offsets and trees.

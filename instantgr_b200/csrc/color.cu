@@ -11,13 +11,27 @@
 //
 // The reference is nondeterministic (a claiming thread re-reads the cell right
 // after its atomicMax while others are still writing, and returns early).
-// Here claiming, committing and blocking are separate phases separated by
-// grid barriers, so the batches depend only on the input.
+// Here claiming and committing are separate phases separated by grid barriers,
+// so the batches depend only on the input.
+//
+// A cell of the map holds the round, the rank of its claimer and, once the
+// claimer has joined, a member bit above both.  A claim of a later round
+// therefore replaces every older one but a member's, so that a blocked net need
+// not look for the cells it still holds to give them back (660M reads on the
+// 800k-net design), a lost net sees from the map alone whether a member owns one
+// of its points, and, since members' cells do not change any more, it claims for
+// the next round in the same phase: two grid barriers a round.  The owners are
+// those of the round-by-round release: a net joins only when no candidate of a
+// higher rank claims its points, candidates only drop out, and so no later claim
+// ever meets a member's cell with a higher rank.  The 800k-net design's four
+// colourings went from 17.4 + 7.5 + 4.5 + 4.0 to 16.2 + 6.2 + 3.5 + 3.1 ms, most
+// of it in the rip-up passes through a warp per net of short lists; what bounds
+// them now is the chain of dependent reads of a phase and the atomics of the claims.
 //
 // Work layout: the cells a net claims are precomputed once (claim lists, CSR
 // per shape) and gathered per rank into one 16-byte header; a group of 8 lanes
-// handles one net.  Each round walks only the nets it concerns: the
-// candidates (claim, commit) and the nets that lost a point (block); the lists
+// handles one net (a warp, when there are few).  Each round walks only the nets it
+// concerns: the candidates (commit) and the nets that lost a point; the lists
 // are rebuilt every phase with one global atomic per block (appends are staged
 // in shared memory).  The whole colouring is one persistent cooperative
 // kernel; the last rounds of a batch, which have few candidates, run in one
@@ -40,22 +54,28 @@ namespace igr {
 namespace {
 
 constexpr int kThreads = 1024;
-constexpr int kG = 8;                          // lanes per net
+constexpr int kG = 8;                          // lanes per net of long lists
 constexpr int kGroups = kThreads / kG;         // groups per block
-constexpr unsigned kGroupMask = (1u << kG) - 1;
 constexpr int kBuf = 4096;                     // staged list entries per block
 // rounds with at most this many candidates run in block 0 alone (two nets per
 // group and phase at most)
 constexpr int kBlockRounds = 2 * kGroups;
 
-// flags (ints): [2] batches, [4] barrier counter, [6] error, [8] rounds run,
-// [9] lost count, [10] next candidate count, [11..12] nets left after a batch
-// (by batch parity)
-enum : int { F_NB = 2, F_BAR = 4, F_ERR = 6, F_ROUNDS = 8, F_LOST = 9, F_CAND = 10, F_LEFT = 11, F_DIRTY = 13 };
+// flags (ints): [0..1] lost counts, [2] batches, [4] barrier counter, [6] error,
+// [8] rounds run, [9..10] candidate counts (both by round parity), [11..12] nets
+// left after a batch (by batch parity), [13] cells to recompute.  A counter is
+// zeroed one phase before it is used and was last read two barriers earlier.
+enum : int { F_LOST = 0, F_NB = 2, F_BAR = 4, F_ERR = 6, F_ROUNDS = 8, F_CAND = 9, F_LEFT = 11, F_DIRTY = 13 };
+
+constexpr int kMaxRounds = 30;
+constexpr int kMember = 1 << 30;
+// map value of net k's claim in an epoch (the round, unless ranks leave too few
+// bits: then the other claims are cleared from time to time)
+__device__ __forceinline__ int claim_value(const ColorDev &c, int epoch, int k) { return epoch << c.rank_bits | k; }
 
 // memory operations of this thread, summed into c.ops at the end (roofline
 // accounting): claimed cells, points checked for commit, points checked for
-// blocking, cells checked for release, list entries scanned
+// blocking, cells checked when a net joins, list entries scanned
 struct Ops {
     unsigned long long claims = 0, points = 0, bpoints = 0, releases = 0, scans = 0;
 };
@@ -121,66 +141,113 @@ __device__ int block_exclusive(int v, int *total) {
 // map and batch change during the kernel: read them from L2
 __device__ __forceinline__ int owner(const ColorDev &c, int cell) { return __ldcg(c.map + cell); }
 
-// Candidates claim their cells, four cells in flight per lane.  Blocks blk,
-// blk+nblk, ... of the workers; group j of a block takes list entry j.
-__device__ __forceinline__ void claim_phase(const ColorDev &c, const int *list, int n, int blk, int nblk, Ops &ops) {
-    const int gl = threadIdx.x % kG;
-    for (int idx = blk * kGroups + threadIdx.x / kG; idx < n; idx += nblk * kGroups) {
+// The three phases of a round.  A group of G lanes takes a net; blocks blk,
+// blk+nblk, ... of the workers, group j of a block list entry j.  Lists that
+// leave warps without a net are walked with a warp per net (a net of 300 claims
+// takes three steps in place of ten), longer ones with kG lanes.
+template <typename F8, typename F32>
+__device__ __forceinline__ void by_length(int n, int nblk, F8 &&f8, F32 &&f32) {
+    if (n <= nblk * (kThreads / 32)) f32();
+    else f8();
+}
+
+// Candidates claim their cells, four cells in flight per lane.  (Reading a cell
+// before the atomic, though most cells have a higher owner already, made the
+// claims 1.4 times slower: the atomics are not waited for, the reads are.)
+template <int G>
+__device__ __forceinline__ void claim_cells(const ColorDev &c, int4 h, int gl, int v) {
+    for (int i = h.x + gl; i < h.y; i += 4 * G) {
+        int cl[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) cl[u] = i + u * G < h.y ? __ldg(c.claim + i + u * G) : -1;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (cl[u] >= 0) atomicMax(c.map + cl[u], v);
+    }
+}
+template <int G>
+__device__ __forceinline__ void claim_nets(const ColorDev &c, const int *list, int n, int blk, int nblk, Ops &ops) {
+    constexpr int kPer = kThreads / G;
+    const int gl = threadIdx.x % G;
+    for (int idx = blk * kPer + threadIdx.x / G; idx < n; idx += nblk * kPer) {
         const int k = list[idx];
         const int4 h = c.hdr[k];
         if (gl == 0) ops.claims += h.y - h.x;
-        for (int i = h.x + gl; i < h.y; i += 4 * kG) {
-            const int c0 = __ldg(c.claim + i);
-            const int c1 = i + kG < h.y ? __ldg(c.claim + i + kG) : -1;
-            const int c2 = i + 2 * kG < h.y ? __ldg(c.claim + i + 2 * kG) : -1;
-            const int c3 = i + 3 * kG < h.y ? __ldg(c.claim + i + 3 * kG) : -1;
-            atomicMax(c.map + c0, k);
-            if (c1 >= 0) atomicMax(c.map + c1, k);
-            if (c2 >= 0) atomicMax(c.map + c2, k);
-            if (c3 >= 0) atomicMax(c.map + c3, k);
-        }
+        claim_cells<G>(c, h, gl, claim_value(c, 0, k));
     }
 }
+// round 0 of a batch
+__device__ __forceinline__ void claim_phase(const ColorDev &c, const int *list, int n, int blk, int nblk, Ops &ops) {
+    by_length(n, nblk, [&] { claim_nets<kG>(c, list, n, blk, nblk, ops); },
+              [&] { claim_nets<32>(c, list, n, blk, nblk, ops); });
+}
 
-// Candidates owning all their points join batch `cur`; the others go to the
-// lost list.  Block-uniform loop (staging and flushes).
-__device__ __forceinline__ void commit_phase(const ColorDev &c, Stage &st, const int *list, int n, int cur,
-                                             int *lost_cnt, int blk, int nblk, Ops &ops) {
-    const int lane = threadIdx.x & 31, grp = lane / kG, gl = lane % kG;
+// Candidates owning all their points join batch `cur` and mark the cells they
+// own; the others go to the lost list.  (Four points in flight per lane made
+// this and the next phase 1.1 times slower, stopping at the first foreign point,
+// G points at a time, 1.4 times: fewer reads, but a longer chain of them.)  Block-uniform loop (staging and flushes).
+template <int G>
+__device__ __forceinline__ void commit_nets(const ColorDev &c, Stage &st, const int *list, int n, int epoch, int cur,
+                                            int *lost_cnt, int blk, int nblk, Ops &ops) {
+    constexpr int kPer = kThreads / G;
+    const int lane = threadIdx.x & 31, grp = lane / G, gl = lane % G;
     int it = 0;
-    for (int b0 = blk * kGroups; b0 < n; b0 += nblk * kGroups, it++) {
-        const int idx = b0 + threadIdx.x / kG;
+    for (int b0 = blk * kPer; b0 < n; b0 += nblk * kPer, it++) {
+        const int idx = b0 + threadIdx.x / G;
         const bool valid = idx < n;
         const int k = valid ? list[idx] : -1;
+        const int v = claim_value(c, epoch, k);
+        int4 h = make_int4(0, 0, 0, 0);
         bool ok = true;
         if (valid) {
-            const int4 h = c.hdr[k];
+            h = c.hdr[k];
             if (gl == 0) ops.points += h.w - h.z;
-            for (int i = h.z + gl; i < h.w; i += 2 * kG) {
+            for (int i = h.z + gl; i < h.w; i += 2 * G) {
                 const int p0 = __ldg(c.pts + i);
-                const int p1 = i + kG < h.w ? __ldg(c.pts + i + kG) : -1;
+                const int p1 = i + G < h.w ? __ldg(c.pts + i + G) : -1;
                 const int o0 = owner(c, p0);
-                const int o1 = p1 >= 0 ? owner(c, p1) : k;
-                ok &= (o0 == k) & (o1 == k);
+                const int o1 = p1 >= 0 ? owner(c, p1) : v;
+                ok &= (o0 == v) & (o1 == v);
             }
         }
-        const unsigned bad = (__ballot_sync(0xffffffffu, !ok) >> (grp * kG)) & kGroupMask;
-        if (valid && bad == 0 && gl == 0) c.batch[k] = cur;
+        const unsigned bad = (__ballot_sync(0xffffffffu, !ok) >> (grp * G)) & (0xffffffffu >> (32 - G));
+        if (valid && bad == 0) {
+            if (gl == 0) {
+                c.batch[k] = cur;
+                ops.releases += h.y - h.x;
+            }
+            for (int i = h.x + gl; i < h.y; i += 4 * G) {
+                int cl[4], ow[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) cl[u] = i + u * G < h.y ? __ldg(c.claim + i + u * G) : -1;
+#pragma unroll
+                for (int u = 0; u < 4; u++) ow[u] = cl[u] >= 0 ? owner(c, cl[u]) : -1;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (ow[u] == v) c.map[cl[u]] = v | kMember;
+            }
+        }
         stage(st, valid && bad != 0 && gl == 0, k, lane);
-        if ((it + 1) % (kBuf / kGroups) == 0) flush(st, c.lost, lost_cnt);
+        if ((it + 1) % (kBuf / kPer) == 0) flush(st, c.lost, lost_cnt);
     }
     flush(st, c.lost, lost_cnt);
 }
+__device__ __forceinline__ void commit_phase(const ColorDev &c, Stage &st, const int *list, int n, int epoch, int cur,
+                                             int *lost_cnt, int blk, int nblk, Ops &ops) {
+    by_length(n, nblk, [&] { commit_nets<kG>(c, st, list, n, epoch, cur, lost_cnt, blk, nblk, ops); },
+              [&] { commit_nets<32>(c, st, list, n, epoch, cur, lost_cnt, blk, nblk, ops); });
+}
 
-// Lost nets with a point owned by a member are blocked and release their
-// cells at once (a blocked net's cells are no member's points, so the release
-// cannot change another net's check); the others stay candidates.
-__device__ __forceinline__ void block_phase(const ColorDev &c, Stage &st, int n, int *cand_cnt, int blk, int nblk,
-                                            Ops &ops) {
-    const int lane = threadIdx.x & 31, grp = lane / kG, gl = lane % kG;
+// Lost nets with a point owned by a member are blocked for this batch; the
+// others stay candidates and claim their cells for the next round, `epoch`.
+template <int G>
+__device__ __forceinline__ void next_nets(const ColorDev &c, Stage &st, int n, int epoch, int *cand_cnt, int blk,
+                                          int nblk, Ops &ops) {
+    constexpr int kPer = kThreads / G;
+    const int lane = threadIdx.x & 31, grp = lane / G, gl = lane % G;
     int it = 0;
-    for (int b0 = blk * kGroups; b0 < n; b0 += nblk * kGroups, it++) {
-        const int idx = b0 + threadIdx.x / kG;
+    for (int b0 = blk * kPer; b0 < n; b0 += nblk * kPer, it++) {
+        const int idx = b0 + threadIdx.x / G;
         const bool valid = idx < n;
         const int k = valid ? c.lost[idx] : -1;
         int4 h = make_int4(0, 0, 0, 0);
@@ -188,64 +255,56 @@ __device__ __forceinline__ void block_phase(const ColorDev &c, Stage &st, int n,
         if (valid) {
             h = c.hdr[k];
             if (gl == 0) ops.bpoints += h.w - h.z;
-            for (int i = h.z + gl; i < h.w; i += 2 * kG) {
+            for (int i = h.z + gl; i < h.w; i += 2 * G) {
                 const int p0 = __ldg(c.pts + i);
-                const int p1 = i + kG < h.w ? __ldg(c.pts + i + kG) : -1;
+                const int p1 = i + G < h.w ? __ldg(c.pts + i + G) : -1;
                 const int o0 = owner(c, p0);
                 const int o1 = p1 >= 0 ? owner(c, p1) : -1;
-                const int b0v = o0 != -1 ? __ldcg(c.batch + o0) : -1;
-                const int b1v = o1 != -1 ? __ldcg(c.batch + o1) : -1;
-                hit |= (b0v != -1) | (b1v != -1);
+                hit |= (o0 >= kMember) | (o1 >= kMember);
             }
         }
-        const bool blocked = ((__ballot_sync(0xffffffffu, hit) >> (grp * kG)) & kGroupMask) != 0;
-        if (valid && blocked) {
-            if (gl == 0) ops.releases += h.y - h.x;
-            for (int i = h.x + gl; i < h.y; i += 4 * kG) {
-                int cl[4], ow[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) cl[u] = i + u * kG < h.y ? __ldg(c.claim + i + u * kG) : -1;
-#pragma unroll
-                for (int u = 0; u < 4; u++) ow[u] = cl[u] >= 0 ? owner(c, cl[u]) : -1;
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-                    if (ow[u] == k) c.map[cl[u]] = -1;
-            }
+        const bool blocked = ((__ballot_sync(0xffffffffu, hit) >> (grp * G)) & (0xffffffffu >> (32 - G))) != 0;
+        if (valid && !blocked) {
+            if (gl == 0) ops.claims += h.y - h.x;
+            claim_cells<G>(c, h, gl, claim_value(c, epoch, k));
         }
         stage(st, valid && !blocked && gl == 0, k, lane);
-        if ((it + 1) % (kBuf / kGroups) == 0) flush(st, c.cand, cand_cnt);
+        if ((it + 1) % (kBuf / kPer) == 0) flush(st, c.cand, cand_cnt);
     }
     flush(st, c.cand, cand_cnt);
 }
+__device__ __forceinline__ void next_phase(const ColorDev &c, Stage &st, int n, int epoch, int *cand_cnt, int blk,
+                                           int nblk, Ops &ops) {
+    by_length(n, nblk, [&] { next_nets<kG>(c, st, n, epoch, cand_cnt, blk, nblk, ops); },
+              [&] { next_nets<32>(c, st, n, epoch, cand_cnt, blk, nblk, ops); });
+}
 
 // Rounds `round`.. of batch `cur` in this block alone, over the nc candidates
-// in c.cand.  Every thread of the block calls it.
+// in c.cand, which have claimed in that round.  Every thread of the block calls it.
 __device__ void block_rounds(const ColorDev &c, Stage &st, int round, int nc, int cur, int *rounds_ctr, Ops &ops) {
     __shared__ int s_lost, s_cand;
-    for (; round < 30; round++) {
+    while (true) {
         if (threadIdx.x == 0) {
             s_lost = 0;
             s_cand = 0;
             (*rounds_ctr)++;
         }
         __syncthreads();
-        claim_phase(c, c.cand, nc, 0, 1, ops);
-        __syncthreads();
-        commit_phase(c, st, c.cand, nc, cur, &s_lost, 0, 1, ops);
+        commit_phase(c, st, c.cand, nc, round, cur, &s_lost, 0, 1, ops);
         const int nl = s_lost;  // flush ends with a block barrier
-        if (nl == nc) break;    // no net joined in this round
-        block_phase(c, st, nl, &s_cand, 0, 1, ops);
+        if (nl == nc || round + 1 >= kMaxRounds) break;
+        round++;
+        next_phase(c, st, nl, round, &s_cand, 0, 1, ops);
         nc = s_cand;
         __syncthreads();  // every thread has read the counters before they are reset
         if (nc == 0) break;
     }
 }
 
-// Per batch: candidates claim (atomicMax of their rank on their claim cells),
-// candidates owning all their points join, lost nets are blocked or stay
-// candidates.  Three grid barriers per round; the last rounds of a batch,
-// with few candidates, run in block 0 alone.  The lists are unordered: every
-// phase is order-independent.
+// Per batch: every net without a batch claims (atomicMax), candidates owning
+// all their points join, lost nets are blocked or claim again.  Two grid
+// barriers per round; the last rounds of a batch, with few candidates, run in
+// block 0 alone.  The lists are unordered: every phase is order-independent.
 __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int max_batches) {
     __shared__ Stage st;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -256,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
     volatile int *vflags = c.flags;
     unsigned *bar = reinterpret_cast<unsigned *>(c.flags + F_BAR);
     int *err = c.flags + F_ERR;
-    unsigned epoch = 0;
+    unsigned epoch_of_bar = 0;
     Ops ops;
     auto sum_ops = [&]() {
         if (!c.ops) return;
@@ -282,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
         c.map[i] = -1;
         if (inc) c.rev_cnt[i] = 0;
     }
-    if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+    if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
     if (inc) {
         // claimers of every cell (ranks), grouped by cell: counts, an exclusive
         // scan over the cells (a chunk per block), then the entries
@@ -290,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
             const int4 h = c.hdr[k];
             for (int i = h.x; i < h.y; i++) atomicAdd(c.rev_cnt + __ldg(c.claim + i), 1);
         }
-        if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+        if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         const int chunk = (XY + gridDim.x - 1) / gridDim.x;
         const int lo = min(XY, blockIdx.x * chunk), hi = min(XY, lo + chunk);
         const int per = (hi - lo + kThreads - 1) / kThreads;
@@ -299,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
         for (int i = a0; i < a1; i++) mine += c.rev_cnt[i];
         int run = block_exclusive(mine, &total);
         if (threadIdx.x == 0) c.part[blockIdx.x] = total;
-        if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+        if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         if (tid == 0) {
             int acc = 0;
             for (int b = 0; b < (int)gridDim.x; b++) {
@@ -308,14 +367,14 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
                 acc += t;
             }
         }
-        if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+        if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         run += c.part[blockIdx.x];
         for (int i = a0; i < a1; i++) {
             c.rev_off[i] = run;
             run += c.rev_cnt[i];
             c.rev_cnt[i] = 0;
         }
-        if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+        if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         for (int k = tid; k < c.n; k += nth) {
             const int4 h = c.hdr[k];
             for (int i = h.x; i < h.y; i++) {
@@ -323,49 +382,54 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
                 c.rev[c.rev_off[cell] + atomicAdd(c.rev_cnt + cell, 1)] = k;
             }
         }
-        if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+        if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
     }
     int na = c.n;
     for (int cur = 0; cur < max_batches; cur++) {
         const int *cand = act;  // round 0: every net without a batch
-        int nc = na;
-        int round = 0;
-        bool tail = false;
-        for (; round < 30; round++) {
-            if (round > 0 && nc <= kBlockRounds) {
-                tail = true;
-                break;
+        int nc = na, epoch = 0;
+        // with the round-0 map kept up to date, round 0 of a later batch starts
+        // from it (its counters were reset before the last barrier)
+        const bool kept = inc && cur > 0;
+        if (!kept) {
+            if (tid == 0) flags[F_LOST] = 0;
+            claim_phase(c, cand, nc, blockIdx.x, gridDim.x, ops);
+            if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
+            if (tid == 0) flags[F_LEFT + ((cur + 1) & 1)] = 0;
+        }
+        if (inc && cur == 0)  // the first round-0 map, whether or not its owners have joined yet
+            for (int i = tid; i < XY; i += nth) {
+                const int v = __ldcg(c.map + i);
+                c.snap[i] = v >= 0 ? v & ~kMember : v;
             }
-            // with the round-0 map kept up to date, round 0 of a later batch
-            // starts from it (its counters were reset before the last barrier)
-            const bool kept = inc && round == 0 && cur > 0;
+        for (int round = 0;; epoch++) {
             if (tid == 0) {
                 flags[F_ROUNDS]++;
-                if (!kept) flags[F_LOST] = 0;
+                flags[F_CAND + ((round + 1) & 1)] = 0;
             }
-            if (!kept) {
-                claim_phase(c, cand, nc, blockIdx.x, gridDim.x, ops);
-                if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
-                if (tid == 0) {
-                    flags[F_CAND] = 0;
-                    if (round == 0) flags[F_LEFT + ((cur + 1) & 1)] = 0;
-                }
+            commit_phase(c, st, cand, nc, epoch, cur, flags + F_LOST + (round & 1), blockIdx.x, gridDim.x, ops);
+            if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
+            const int nl = vflags[F_LOST + (round & 1)];
+            if (nl == nc || round + 1 >= kMaxRounds) break;  // no net joined, or the last round
+            round++;
+            if ((epoch + 1) >> (30 - c.rank_bits)) {  // out of epochs: clear all claims but the members'
+                for (int i = tid; i < XY; i += nth)
+                    if (__ldcg(c.map + i) < kMember) c.map[i] = -1;
+                epoch = -1;
+                if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
             }
-            if (inc && round == 0 && cur == 0)  // the first round-0 map, before any release
-                for (int i = tid; i < XY; i += nth) c.snap[i] = __ldcg(c.map + i);
-            commit_phase(c, st, cand, nc, cur, flags + F_LOST, blockIdx.x, gridDim.x, ops);
-            if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
-            const int nl = vflags[F_LOST];
-            if (nl == nc) break;  // no net joined in this round
-            block_phase(c, st, nl, flags + F_CAND, blockIdx.x, gridDim.x, ops);
-            if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+            if (tid == 0) flags[F_LOST + (round & 1)] = 0;
+            next_phase(c, st, nl, epoch + 1, flags + F_CAND + (round & 1), blockIdx.x, gridDim.x, ops);
+            if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
             cand = c.cand;
-            nc = vflags[F_CAND];
+            nc = vflags[F_CAND + (round & 1)];
             if (nc == 0) break;
-        }
-        if (tail) {
-            if (blockIdx.x == 0) block_rounds(c, st, round, nc, cur, flags + F_ROUNDS, ops);
-            if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+            // the tail counts its rounds as epochs
+            if (nc <= kBlockRounds && epoch + 1 == round && !(kMaxRounds >> (30 - c.rank_bits))) {
+                if (blockIdx.x == 0) block_rounds(c, st, round, nc, cur, flags + F_ROUNDS, ops);
+                if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
+                break;
+            }
         }
         // nets still without a batch stay active; the map is cleared for the
         // next batch, or, when the round-0 map is kept, the cells whose
@@ -393,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
             if ((it + 1) % (kBuf / kThreads) == 0) flush(st, act2, flags + F_LEFT + (cur & 1));
         }
         flush(st, act2, flags + F_LEFT + (cur & 1));
-        if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+        if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         na = vflags[F_LEFT + (cur & 1)];
         int *t = act; act = act2; act2 = t;
         if (na == 0) {
@@ -430,15 +494,14 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
                     c.snap[cell] = best;
                 }
             }
-            if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+            if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
             for (int i = tid; i < XY; i += nth) c.map[i] = c.snap[i];
             if (tid == 0) {  // counters of round 0 of the next batch
                 flags[F_DIRTY] = 0;
                 flags[F_LOST] = 0;
-                flags[F_CAND] = 0;
                 flags[F_LEFT + ((cur + 2) & 1)] = 0;
             }
-            if (!grid_sync(bar, err, epoch, c.wait_ns, c.phantom)) return;
+            if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         }
     }
     if (tid == 0) flags[F_NB] = max_batches;
@@ -497,6 +560,7 @@ int run_coloring(ColorDev &c, int max_batch, cudaStream_t s) {
     if (blocks < 1) blocks = 1;
     c.wait_ns = (unsigned long long)test_hooks().wait_ns.load();
     c.phantom = (unsigned)test_hooks().barrier_phantom.load();
+    for (c.rank_bits = 25; c.rank_bits < 29 && (c.n >> c.rank_bits) != 0;) c.rank_bits++;
     cudaMemsetAsync(c.flags, 0, 16 * sizeof(int), s);
     cudaMemsetAsync(c.batch, 0xff, sizeof(int) * (size_t)c.n, s);
     int max_batches = c.n + 1;

@@ -354,10 +354,11 @@ struct ColorDev {
     int *active = nullptr, *active2 = nullptr, *cand = nullptr, *lost = nullptr;
     int4 *hdr = nullptr;      // [n] per rank: claim begin/end, point begin/end
     // optional [5] operation counts, accumulated: claimed cells, commit point
-    // checks, blocking point checks, release checks, list entries scanned
+    // checks, blocking point checks, cells checked when a net joins, list entries scanned
     unsigned long long *ops = nullptr;
     int *flags = nullptr;     // [16] device flags
     int rounds = 0;           // out: colouring rounds run
+    int rank_bits = 25;       // bits of a rank in the map (set by run_coloring)
     // optional (all or none): the round-0 map of every batch kept up to date
     // instead of re-claimed.  rev_off/rev_cnt [X*Y]: claimers of each cell in
     // rev[] (ranks; [total claims]); snap/dirty [X*Y]; part [1024]

@@ -1825,9 +1825,9 @@ void Router::compute_score() {
         for (size_t i = 0; i < d.sel.size(); i++) pin_vias += d.sel[i] < d.X * d.Y;
     }
     // per claimed cell: 4-byte index + 8-byte read-modify-write; per point check:
-    // index + owner (+ batch of the owner when blocking); per release check:
-    // index + owner; per list entry scanned: entry + batch
-    color_bytes = 12.0 * cops[0] + 8.0 * cops[1] + 12.0 * cops[2] + 8.0 * cops[3] + 8.0 * cops[4];
+    // index + owner; per cell checked when a net joins: index + owner; per list
+    // entry scanned: entry + batch
+    color_bytes = 12.0 * cops[0] + 8.0 * cops[1] + 8.0 * cops[2] + 8.0 * cops[3] + 8.0 * cops[4];
     cost_cells = h[2];
     commit_cells = h[3];
     commit_refresh_cells = h[4];
