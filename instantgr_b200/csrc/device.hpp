@@ -212,9 +212,10 @@ struct ShapeArgs {
 };
 void launch_shape_count(const ShapeArgs &a, int *pt_off, int *claim_off, long long *totals, cudaStream_t s);
 // pt_n / claim_n (optional, [n]): per shape the number of distinct points and
-// claimed cells, which the fill sorts and moves to the front of each range
+// claimed cells, which the fill keeps once, at the front of each range (with
+// `big`, [n + 1] ints of scratch); else every repetition is kept
 void launch_shape_fill(const ShapeArgs &a, const int *pt_off, const int *claim_off, int *pts, int *claim,
-                       int *pt_n, int *claim_n, cudaStream_t s);
+                       int *pt_n, int *claim_n, int *big, cudaStream_t s);
 
 // ---- detour DAGs on the device (dagbuild.cu)
 // slice sizes of one builder thread's work area: tree nodes, stem entries,

@@ -473,7 +473,8 @@ void Router::device_shapes(const ShapeArgs &a, ShapeDev &sd) {
         sd.pt_n.release();
         sd.claim_n.release();
     }
-    launch_shape_fill(a, sd.pt_off.p, sd.claim_off.p, sd.pts.p, sd.claim.p, sd.pt_n.p, sd.claim_n.p, s);
+    d_shape_big.alloc((size_t)a.n + 1);
+    launch_shape_fill(a, sd.pt_off.p, sd.claim_off.p, sd.pts.p, sd.claim.p, sd.pt_n.p, sd.claim_n.p, d_shape_big.p, s);
     if (verbose) {
         long long m = 0, us = 0, tr = 0;
         dev_alloc_stats(&m, &us, &tr);

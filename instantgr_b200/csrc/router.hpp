@@ -358,6 +358,7 @@ struct Router {
     void ensure_device();
     void device_shapes(const ShapeArgs &a, ShapeDev &sd);
     DevBuf<long long> d_shape_tot;
+    DevBuf<int> d_shape_big;  // shapes too large for a warp
     DevBuf<int> d2_ptoff, d2_pts, d2_ids;  // DAG points and net ids of the rerouted nets
     // device DAG construction: trees in adjacency order (positions, neighbour
     // lists), the builder, kept nets and the batch layout of the gather
