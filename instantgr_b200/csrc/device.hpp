@@ -210,7 +210,10 @@ struct ShapeArgs {
     int ext_stride = 1;
     int n = 0, X = 0, Y = 0, sparsity = 15;
 };
-void launch_shape_count(const ShapeArgs &a, int *pt_off, int *claim_off, long long *totals, cudaStream_t s);
+// (sums: 2 * max(1, shape_count_blocks(n)) entries of scratch)
+int shape_count_blocks(int n);
+void launch_shape_count(const ShapeArgs &a, int *pt_off, int *claim_off, long long *totals, long long *sums,
+                        cudaStream_t s);
 // pt_n / claim_n (optional, [n]): per shape the number of distinct points and
 // claimed cells, which the fill keeps once, at the front of each range (with
 // `big`, [n + 1] ints of scratch); else every repetition is kept

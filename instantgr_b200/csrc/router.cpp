@@ -458,7 +458,8 @@ void Router::device_shapes(const ShapeArgs &a, ShapeDev &sd) {
     sd.claim_off.alloc((size_t)a.n + 1);
     d_shape_tot.alloc(2);
     const double t0 = now_s();
-    launch_shape_count(a, sd.pt_off.p, sd.claim_off.p, d_shape_tot.p, s);
+    d_shape_sums.alloc(2 * (size_t)std::max(1, shape_count_blocks(a.n)));
+    launch_shape_count(a, sd.pt_off.p, sd.claim_off.p, d_shape_tot.p, d_shape_sums.p, s);
     long long h_tot[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(h_tot, d_shape_tot.p, sizeof h_tot, cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "shape counts");

@@ -357,7 +357,7 @@ struct Router {
     const int *route_of(int net) const { return h_routes_ptr + h_route_at[net]; }
     void ensure_device();
     void device_shapes(const ShapeArgs &a, ShapeDev &sd);
-    DevBuf<long long> d_shape_tot;
+    DevBuf<long long> d_shape_tot, d_shape_sums;
     DevBuf<int> d_shape_big;  // shapes too large for a warp
     DevBuf<int> d2_ptoff, d2_pts, d2_ids;  // DAG points and net ids of the rerouted nets
     // device DAG construction: trees in adjacency order (positions, neighbour
