@@ -312,7 +312,7 @@ int igr_dag_route(igr_ctx *c, int n, const int32_t *node_off, const int32_t *nod
 int igr_build_dag(int X, int Y, int mode, int ntree, const int32_t *pos, const int32_t *adj_off, const int32_t *adj,
                   const float *xsum, const float *ysum, int32_t *out, int64_t cap, int64_t *len);
 
-/* Detour DAGs of n trees built on the device, one thread per tree (the
+/* Detour DAGs of n trees built on the device, a warp per tree (the
  * construction of igr_build_dag, which it replaces for the rip-up passes of
  * the router: Lshape_route_detour.hpp:702-748 calls
  * net::generate_detours_reconstruct, src/database_cuda.hpp:1429-2086, per

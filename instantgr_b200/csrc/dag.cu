@@ -699,6 +699,17 @@ void dag_levels(int n, const int *node_off, const int *depth, std::vector<int> &
     }
 }
 
+namespace {
+
+int max_block_smem() {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    return v;
+}
+
+}  // namespace
+
 int launch_dag_route(const GridDev &g, const DagBatchDev &b, int stamp, cudaStream_t s, cudaStream_t aux,
                      cudaEvent_t fork, cudaEvent_t join, int split_nets, int stage_nodes) {
     if (b.n_nodes <= 0 || b.n_nets <= 0) return 0;
@@ -719,7 +730,7 @@ int launch_dag_route(const GridDev &g, const DagBatchDev &b, int stamp, cudaStre
     const int cap_n = b.offers && g.X <= kStageMaxSide && g.Y <= kStageMaxSide ? std::max(0, stage_nodes) : 0;
     auto fit = [&](int n, int m, int warps) -> int {
         if (!cap_n || n <= 0) return 0;
-        const size_t room = (size_t)dag_solo_smem_limit() - sizeof(NodeScratch) * warps;
+        const size_t room = (size_t)max_block_smem() - sizeof(NodeScratch) * warps;
         const int nn = (std::min(n, cap_n) + 31) / 32 * 32, mm = (std::min(m, 2 * nn) + 63) / 64 * 64;
         return (int)std::min(staged_bytes(nn, mm, mm), room);
     };

@@ -1,5 +1,5 @@
-// Host side of the device DAG builder: work-area size classes, the size and
-// write passes, and the layout of the per-DAG arrays.
+// Host side of the device DAG builder: work-area size classes and the pools of
+// the finished DAGs.
 #include <algorithm>
 
 #include "router.hpp"
@@ -8,43 +8,18 @@ namespace igr {
 
 namespace {
 
-// Work-area slices per size class and the most builders a class runs;
-// most DAGs fit the first class (nets of up to 12 pins give trees of at most
-// 22 nodes), the few larger ones the second, whose builders keep their work
-// area in shared memory, one per SM; the third is for split nets whose trees
-// kept growing.
-struct DagClass {
-    DagCaps caps;
-    int threads;
-    bool solo;  // one builder per block
-};
-const DagClass kClasses[] = {
-    {{32, 256, 256, 256, 512, 1024}, 148 * 512, false},
-    {{128, 1024, 1024, 1536, 3072, 6144}, 148, true},
-    {{2048, 16384, 16384, 16384, 32768, 65536}, 512, true},
-};
+// Size classes of the work area: most DAGs fit the first (nets of up to 12 pins
+// give trees of at most 22 nodes), the few larger ones the second, both a warp
+// per net in shared memory; the third, in global memory, is for split nets whose
+// trees kept growing.
 constexpr int kNumClasses = 3;
-
-int round_threads(int n, int cap) {
-    const int t = std::min(cap, std::max(n, 1));
-    return (t + 127) / 128 * 128;
-}
+constexpr int kLastBuilders = 512;
 
 void run_class(DeviceDags &d, DagBuildArgs a, int cls, const std::vector<int> &members, cudaStream_t s) {
-    const DagClass &c = kClasses[cls];
     const int n = (int)members.size();
     if (n == 0) return;
-    const long long per = dag_work_ints(c.caps);
-    const bool in_smem = c.solo && per * 4 <= dag_solo_smem_limit();
-    const int threads = c.solo ? std::min(n, c.threads) : round_threads(n, c.threads);
-    a.caps = c.caps;
-    if (in_smem) {
-        a.work = nullptr;
-    } else {
-        d.work.alloc((size_t)threads * (size_t)per);
-        a.work = d.work.p;
-    }
     a.n_list = n;
+    a.queue = d.queue.p;
     bool identity = true;  // 0 .. n-1 in order
     for (int i = 0; i < n && identity; i++) identity = members[i] == i;
     if (identity) {
@@ -53,10 +28,13 @@ void run_class(DeviceDags &d, DagBuildArgs a, int cls, const std::vector<int> &m
         d.list.upload(members, s);
         a.list = d.list.p;
     }
-    if (c.solo)
-        launch_dag_build_solo(a, threads, s);
-    else
-        launch_dag_build(a, threads, s);
+    const int builders = std::min(n, kLastBuilders);
+    a.work = nullptr;
+    if (cls == kNumClasses - 1) {
+        d.work.alloc((size_t)builders * dag_work_bytes());
+        a.work = d.work.p;
+    }
+    launch_dag_build(a, cls, builders, s);
     cuda_check(cudaGetLastError(), "DAG build launch");
 }
 
@@ -72,7 +50,7 @@ void grow_keep(DevBuf<int> &b, size_t count, size_t keep, cudaStream_t s) {
 
 }  // namespace
 
-void DeviceDags::build(DagBuildArgs a, cudaStream_t s, const std::vector<int> *order_key) {
+void DeviceDags::build(DagBuildArgs a, cudaStream_t s) {
     const int n = a.n_list;
     hs.assign((size_t)n * kDagSizeFields, 0);
     tier.assign(n, 0);
@@ -80,6 +58,7 @@ void DeviceDags::build(DagBuildArgs a, cudaStream_t s, const std::vector<int> *o
     sizes.alloc((size_t)n * kDagSizeFields);
     node_at.alloc(n); edge_at.alloc(n); point_at.alloc(n);
     used.alloc(3);
+    queue.alloc(1);
     cuda_check(cudaMemsetAsync(used.p, 0, 3 * sizeof(unsigned long long), s), "memset");
     // pools sized from the last build's entries per DAG, with a margin
     auto want = [&](double per) { return (size_t)(per * 1.25 * n) + 4096; };
@@ -97,12 +76,6 @@ void DeviceDags::build(DagBuildArgs a, cudaStream_t s, const std::vector<int> *o
     set_pools();
     std::vector<int> members(n), next;  // DAGs to build in this class; for the next class
     for (int k = 0; k < n; k++) members[k] = k;
-    // builders of nets alike in size side by side: a warp's 32 builders then
-    // walk loops of similar lengths and diverge less (c2: 21/18/18 -> 18/13/13
-    // ms per pass); each DAG is built alone, so the DAGs do not change
-    if (order_key)
-        std::stable_sort(members.begin(), members.end(),
-                         [&](int l, int r) { return (*order_key)[l] > (*order_key)[r]; });
     int cls = 0, regrow = 0;
     while (true) {
         run_class(*this, a, cls, members, s);

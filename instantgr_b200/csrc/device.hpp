@@ -221,11 +221,6 @@ void launch_shape_fill(const ShapeArgs &a, const int *pt_off, const int *claim_o
                        int *pt_n, int *claim_n, int *big, cudaStream_t s);
 
 // ---- detour DAGs on the device (dagbuild.cu)
-// slice sizes of one builder thread's work area: tree nodes, stem entries,
-// mirror entries, DAG nodes, links, conflict points (before deduplication)
-struct DagCaps {
-    int tc = 32, sc = 512, mc = 512, nc = 512, ec = 1024, pc = 2048;
-};
 constexpr int kDagSizeFields = 7;  // per DAG: nodes, links, points, depth levels, child slots, widest slot, status
 struct DagBuildArgs {
     int n_list = 0;
@@ -237,8 +232,8 @@ struct DagBuildArgs {
     const int *adj = nullptr;       // neighbours (net-local indices)
     const float *xsum = nullptr, *ysum = nullptr;  // congestion view [X][Y]
     int X = 0, Y = 0, mode = 2;
-    DagCaps caps;
-    int *work = nullptr;            // threads x dag_work_ints(caps)
+    unsigned char *work = nullptr;  // class 2: builders x dag_work_bytes()
+    int *queue = nullptr;           // work counter
     int *sizes = nullptr;           // [k][kDagSizeFields]; status 1: work area too small, 2: malformed, 3: pool full
     long long *node_at = nullptr, *edge_at = nullptr, *point_at = nullptr;  // [k] where DAG k was placed
     // pools: entries used so far (nodes, edges, points) and their capacities
@@ -247,12 +242,12 @@ struct DagBuildArgs {
     int *out_nodes = nullptr, *out_par_num = nullptr, *out_child_num = nullptr, *out_depth = nullptr;
     int *out_par = nullptr, *out_child_idx = nullptr, *out_points = nullptr;
 };
-long long dag_work_ints(const DagCaps &c);
-void launch_dag_build(const DagBuildArgs &a, int threads, cudaStream_t s);
-// one builder per block: work area in shared memory (a.work null, at most
-// dag_solo_smem_limit() bytes) or in global memory (builders x slices)
-void launch_dag_build_solo(const DagBuildArgs &a, int builders, cudaStream_t s);
-int dag_solo_smem_limit();
+// Grids of at most this many GCells a side: 16-bit work areas.
+constexpr int kDagNarrowSide = 1 << 14;
+size_t dag_work_bytes();
+// class 0 (small DAGs), 1 (larger ones): work areas in shared memory; 2: in
+// global memory, `builders` of them
+void launch_dag_build(const DagBuildArgs &a, int cls, int builders, cudaStream_t s);
 // batch layout: per net (in batch order) its DAG k, batch-local node base,
 // edge base, slot base, level base, position in the batch and batch; per
 // batch its first node, edge, node+1, level and net entries and first net

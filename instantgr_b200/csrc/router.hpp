@@ -126,7 +126,8 @@ struct DagBatchInfo {
 // area are built again with larger slices; DAGs that find a pool full are
 // built again after the pools have grown (keeping what they hold).
 struct DeviceDags {
-    DevBuf<int> work, sizes, list;
+    DevBuf<unsigned char> work;
+    DevBuf<int> sizes, list, queue;
     DevBuf<long long> node_at, edge_at, point_at;
     DevBuf<unsigned long long> used;
     DevBuf<int> nodes, par_num, child_num, depth, par, child_idx, points;
@@ -135,9 +136,7 @@ struct DeviceDags {
     std::vector<int> tier;  // work-area size class each DAG fits
     // a.ids, a.n_list and the tree, congestion and grid fields set; the rest
     // is filled in here
-    // order_key (optional, per DAG): the first class builds its DAGs in
-    // descending key order
-    void build(DagBuildArgs a, cudaStream_t s, const std::vector<int> *order_key = nullptr);
+    void build(DagBuildArgs a, cudaStream_t s);
     int sz(int k, int f) const { return hs[(size_t)k * kDagSizeFields + f]; }
 };
 

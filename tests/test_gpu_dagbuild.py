@@ -78,6 +78,47 @@ def test_device_dags_match_host_builder(mode, seed, max_pins, density):
         assert np.array_equal(recs[off[k]:off[k + 1]], want), f"tree {k}"
 
 
+@pytest.mark.parametrize("T,X,Y", [(2, 700, 500), (32, 700, 500), (33, 700, 500), (128, 700, 500), (129, 700, 500),
+                                   (400, 700, 500), (32, 16384, 8), (12, 16385, 8), (60, 8, 16385), (200, 16500, 6)])
+def test_device_dags_at_class_edges(T, X, Y):
+    """Trees at the node limits of the work-area classes, and grids on both sides
+    of the limit of the packed positions: the host builder's records.  Trees of
+    400 nodes give more than the largest work area takes, and are refused."""
+    rng = np.random.default_rng(100 + T)
+    tree_off, pos, adj_off, adj = [0], [], [0], []
+    for _ in range(12):
+        xs, ys = [int(rng.integers(X))], [int(rng.integers(Y))]
+        nb = [[] for _ in range(T)]
+        for v in range(1, T):
+            p = int(rng.integers(max(0, v - 4), v))
+            step = int(rng.choice([3, 30, 160]))
+            x = int(np.clip(xs[p] + rng.integers(-step, step + 1), 0, X - 1))
+            y = int(np.clip(ys[p] + rng.integers(-step, step + 1), 0, Y - 1))
+            if rng.random() < 0.3:
+                x, y = (xs[p], y) if rng.random() < 0.5 else (x, ys[p])
+            xs.append(x)
+            ys.append(y)
+            nb[v].append(p)
+            nb[p].append(v)
+        for v in range(T):
+            lay = int(rng.integers(0, 10))
+            pos.append(lay * X * Y + xs[v] * Y + ys[v])
+            adj.extend(nb[v])
+            adj_off.append(len(adj))
+        tree_off.append(len(pos))
+    xsum, ysum = _view(rng, X, Y, 0.02)
+    pos, adj_off, adj = (np.array(v, np.int32) for v in (pos, adj_off, adj))
+    if T == 400:  # more nodes, links or points than the largest work area has
+        with pytest.raises(ig.IgrError, match="CAPACITY"):
+            ig.build_dags(X, Y, 0, tree_off, pos, adj_off, adj, xsum, ysum)
+        return
+    recs, off = ig.build_dags(X, Y, 0, tree_off, pos, adj_off, adj, xsum, ysum)
+    for k in range(len(tree_off) - 1):
+        a, b = tree_off[k], tree_off[k + 1]
+        want = ig.build_dag(X, Y, 0, pos[a:b], adj_off[a:b + 1] - adj_off[a], adj[adj_off[a]:adj_off[b]], xsum, ysum)
+        assert np.array_equal(recs[off[k]:off[k + 1]], want), f"tree {k}"
+
+
 def test_device_dags_reject_bad_trees():
     X, Y = 50, 50
     xs, ys = np.zeros(X * Y, np.float32), np.zeros(X * Y, np.float32)
