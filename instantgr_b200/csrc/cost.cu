@@ -3,19 +3,16 @@
 //
 // Replaces three full-grid kernels of InstantGR (update_wcost_cuda_ispd24,
 // update_vcost_ispd24, compute_presum; src/graph.hpp:40-71, :101-104,
-// :405-430).  One CTA of 256 threads owns one track: it stages the track's
-// capacity and demand in shared memory with coalesced loads, evaluates the
-// cost model for every cell, writes vcost (f32), and scans the wire costs in
-// f64 into presum.  The wire cost array itself is never written: 20 bytes of
-// DRAM traffic per cell (4+4 read, 4+8 written) instead of the reference's
-// >= 44.
+// :405-430).  One CTA owns one track, a warp of it 256 consecutive cells: it
+// loads capacity and demand, evaluates the cost model for every cell, writes
+// vcost (f32), and scans the wire costs in f64 into presum.  The wire cost array
+// itself is never written: 20 bytes of DRAM traffic per cell (4+4 read, 4+8
+// written) instead of the reference's >= 44.
 //
 // The prefix sum keeps the exact association of the reference's in-place
 // Sklansky scan (at level d, element i with bit d set adds element
 // ((i >> d) << d) - 1), so presum is bit-identical to the reference's for the
-// same demand.  Element i sits at thread i % 256, row i / 256: levels 0-4 are
-// lane shuffles, levels 5-7 go through shared memory between warps, and levels
-// >= 8 combine whole rows, whose running totals every thread tracks itself.
+// same demand.
 #include "kcommon.cuh"
 #include "host.hpp"
 
@@ -26,8 +23,6 @@
 namespace igr {
 
 namespace {
-
-constexpr int kTrackThreads = 256;
 
 // Cost model of cell i of a track staged in s_cap / s_dem: writes its via cost
 // and returns the scan input, the wire cost of edge i-1 (0 for i = 0).
@@ -65,133 +60,220 @@ __device__ __forceinline__ double cell_costs(const GridDev &g, const TrackInfo &
 // reference's exponent arguments 0.5 * (d - c) and 1.5 * d are formed in
 // double from float operands, where both products are exact, and rounded to
 // float, which is the correctly rounded float product 0.5f * (d - c) or
-// 1.5f * d; the comparison with 0.001 stays in double.
-__device__ __forceinline__ float of_cost_f(bool has_cap, float c, float d) {
-    if (has_cap) return __expf(0.5f * (d - c));
-    return d > 0.f ? __expf(1.5f * d) : 0.f;
+// 1.5f * d.  Its test c > 0.001 in double is c >= 0.001f (the least float above
+// it), and (float)((double)d + 0.5) and + 1.0 are the float sums (rounding the sum of
+// two floats to double first never changes its rounding to float).
+//
+// float to double by the integer multiplier, for normal floats and, up to an
+// error of 2^-127, zero
+__device__ __forceinline__ double widen(float f) {
+    return __longlong_as_double((long long)((unsigned long long)__float_as_uint(f) * 0x20000000ull + (0x38000000ull << 32)));
+}
+// A cell's costs of one more unit (rounded to float, its only use) and of half a
+// unit (graph.hpp:40-71).  The conversions to double are what the refresh has most
+// of on the slowest pipe, so the usual ones go through the multiplier: without
+// capacity a cost is 0 or at least 1, so that 2^-127 is rounded away or cancels;
+// with capacity the costs have to be well above it.
+__device__ __forceinline__ void unit_costs(float c, float d, double sc, float &one, double &half) {
+    const bool has_cap = c >= 0.001f;
+    const float off = has_cap ? c : 0.f, k = has_cap ? 0.5f : 1.5f;
+    const float d5 = d + 0.5f, d1 = d + 1.f;
+    const float e0 = has_cap || d > 0.f ? __expf(k * (d - off)) : 0.f;
+    const float e5 = has_cap || d5 > 0.f ? __expf(k * (d5 - off)) : 0.f;
+    const float e1 = has_cap || d1 > 0.f ? __expf(k * (d1 - off)) : 0.f;
+    double w0 = widen(e0), w5 = widen(e5), w1 = widen(e1);
+    if ((has_cap && e0 < 0x1p-60f) || !(e1 < INFINITY)) {
+        w0 = (double)e0;
+        w5 = (double)e5;
+        w1 = (double)e1;
+    }
+    const double h = (w5 - w0) * sc, o = (w1 - w0) * sc;  // min(1e12, .), 1e12 for NaN
+    half = h < 1e12 ? h : 1e12;
+    one = (float)(o < 1e12 ? o : 1e12);
 }
 
-// Cost model and Sklansky prefix sums of one track of n cells whose capacity
-// and demand are staged in s_cap / s_dem (and s_of1 has room for n floats);
-// every thread of the block calls it and tallies n in g.stats[slot].  Cell i lives at thread i % T, row i / T.
+// Cells of a track by thread: a warp has 128 consecutive ones, or 256 in two
+// passes, four consecutive ones a lane and pass, so that whole sectors are read and
+// written where tracks start on 16 bytes, two levels of the scan are within a lane,
+// and the block has one barrier.  Bound by the instructions of the cost model
+// (81% of the issue slots; 9 of about 150 per cell go to the slowest pipe,
+// exponentials and conversions).  1600 x 1600 cells, 9 layers: 153 us; 840 x 1140:
+// 72; as rows of 256 cells with the costs in shared memory and ten barriers a track
+// 185 and 81.  (Predicated additions in the scan, end cells apart from the others
+// and a path for cells with capacity alone took fewer instructions but 164 to 172 us.)
+constexpr int kPassCells = 128;
+constexpr int kOnePassCells = 1024;  // tracks of at most this many cells: one pass a warp
+template <int P>
+struct TrackCells {
+    float c[P][4], d[P][4];
+};
+
+__device__ __forceinline__ void store_sums(double *p, int left, bool vec, const double (&x)[4], double *stage,
+                                           int lane) {
+    if (vec) {  // lanes past the track's end but for its last cells
+        if (left >= 4) {
+            asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x[0]), "d"(x[1]), "d"(x[2]), "d"(x[3])
+                         : "memory");
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (j < left) p[j] = x[j];
+        }
+        return;
+    }
+    // coalesced through shared memory
+#pragma unroll
+    for (int j = 0; j < 4; j++) stage[4 * lane + j] = x[j];
+    __syncwarp();
+    double *row = p - 4 * lane;
+    const int n = left + 4 * lane;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (32 * j + lane < n) row[32 * j + lane] = stage[32 * j + lane];
+    __syncwarp();
+}
+
+__device__ __forceinline__ double int_to_double(int v) {  // 2^52 + 2^31 + v, less the constant
+    return __hiloint2double(0x43300000, v ^ (int)0x80000000) - 4503601774854144.0;
+}
+
+// Cost model and Sklansky prefix sums of one track of n cells; every thread of
+// the block calls it and tallies n in g.stats[slot].  (pc, pd): capacity and demand
+// of the cell before the warp's first, for lane 0.
 //
-// Each cell's overflow costs at demand d, d + 0.5 and d + 1 are evaluated once
-// and left in shared memory (over its staged capacity and demand), so that
-// cell i reads its left neighbour's instead of evaluating them again:
-// vcost(i) needs the half-unit costs of cells i-1 and i, the wire cost of edge
-// i-1 the unit cost of cell i-1 (graph.hpp:40-71).
-template <int T, int MAXE>
-__device__ __forceinline__ void refresh_track(const GridDev &g, const TrackInfo &ti, float *s_cap, float *s_dem,
-                                              float *s_of1, int slot) {
-    constexpr int W = T / 32;
-    const int n = ti.len;
-    const int E = (n + T - 1) / T;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// Level m of the scan adds element ((i >> m) << m) - 1 to the elements i with bit m
+// set: levels 0-1 within a lane, 2-6 between lanes (the source is a lane's last
+// element), 7 between the two passes, and 8 on between warps, each of which adds
+// up the totals it needs in the order of the levels.
+template <int W, int P>
+__device__ __forceinline__ void refresh_track(const GridDev &g, const TrackInfo &ti, const TrackCells<P> &t, float pc,
+                                              float pd, bool vec, int slot) {
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ double s_total[W];
+    __shared__ double s_stage[W][kPassCells];
+    const int n = ti.len, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double sc = g.short_cost[ti.l];
     const int *elen = ti.dir ? g.ylen : g.xlen;
-    __shared__ double s_wt[W][MAXE];
-    __shared__ double s_rt[MAXE];
-    if (tid == 0) atomicAdd(&g.stats[slot], (unsigned long long)n);  // refreshed cells, for the roofline
-
+    const bool evec = (reinterpret_cast<uintptr_t>(elen) & 15) == 0;
+    if (threadIdx.x == 0) atomicAdd(&g.stats[slot], (unsigned long long)n);  // refreshed cells, for the roofline
+    const bool via_float = (double)(float)g.unit_via == g.unit_via;  // then the float sum is the same
+    double x[P][4];
+    float left_one = 0.f;  // of the cell before this lane's first
+    double left_half = 0.0;
+    if (lane == 0) unit_costs(pc, pd, sc, left_one, left_half);
 #pragma unroll
-    for (int r = 0; r < MAXE; r++) {
-        const int i = tid + r * T;
-        if (r < E && i < n) {
-            const float c = s_cap[i], d = s_dem[i];
-            const bool has_cap = (double)c > 0.001;
-            const double dd = (double)d;
-            s_cap[i] = of_cost_f(has_cap, c, d);
-            s_dem[i] = of_cost_f(has_cap, c, (float)(dd + 0.5));
-            s_of1[i] = of_cost_f(has_cap, c, (float)(dd + 1.0));
+    for (int p = 0; p < P; p++) {
+        const int i0 = warp * P * kPassCells + p * kPassCells + 4 * lane;
+        float one[4];
+        double half[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) unit_costs(t.c[p][j], t.d[p][j], sc, one[j], half[j]);
+        int el[4];
+        load4(elen + i0, n - 1 - i0, evec, el);
+        const float so = __shfl_sync(kFull, one[3], (lane + 31) & 31);
+        const double sh = __shfl_sync(kFull, half[3], (lane + 31) & 31);
+        int se = __shfl_up_sync(kFull, el[3], 1);
+        if (lane == 0) se = i0 > 0 && i0 < n ? elen[i0 - 1] : 0;
+        float po = lane ? so : left_one;
+        double ph = lane ? sh : left_half;
+        if (lane == 0) {  // the second pass follows the first's last lane
+            left_one = so;
+            left_half = sh;
         }
-    }
-    __syncthreads();
-    double x[MAXE];
+        float v[4];
 #pragma unroll
-    for (int r = 0; r < MAXE; r++) {
-        x[r] = 0;
-        const int i = tid + r * T;
-        if (r < E && i < n) {
-            const double of0 = (double)s_cap[i];
-            const double bh = fmin(1e12, ((double)s_dem[i] - of0) * sc);
-            float v;
-            if (i == 0) {
-                v = (float)fmin(1e12, ((double)s_of1[0] - of0) * sc);
-            } else {
-                const double ofp = (double)s_cap[i - 1];
-                const double a1p = fmin(1e12, ((double)s_of1[i - 1] - ofp) * sc);
-                if (i == n - 1) {
-                    v = (float)a1p;
-                } else {
-                    const double bhp = fmin(1e12, ((double)s_dem[i - 1] - ofp) * sc);
-                    v = (float)(bh + bhp);
-                }
-                // scan input: wire cost of edge i-1 (graph.hpp:44-46)
-                float w = (float)a1p;
-                w = (float)fma(g.unit_wire, (double)elen[i - 1], (double)w);
-                x[r] = (double)w;
-            }
-            v = (float)((double)v + g.unit_via);
-            g.vcost[ti.base + i] = v;
+        for (int j = 0; j < 4; j++) {
+            const int i = i0 + j;
+            const float c = i == 0 ? one[0] : i == n - 1 ? po : (float)(half[j] + ph);
+            v[j] = via_float ? c + (float)g.unit_via : (float)((double)c + g.unit_via);
+            // scan input: wire cost of edge i-1 (graph.hpp:44-46)
+            const float w = (float)fma(g.unit_wire, int_to_double(j ? el[j - 1] : se), (double)po);
+            x[p][j] = i > 0 && i < n ? (double)w : 0.0;
+            po = one[j];
+            ph = half[j];
         }
-    }
-    // ---- Sklansky levels 0..4: lanes
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const int src = ((lane >> m) << m) - 1;
-        const bool take = (lane >> m) & 1;
-#pragma unroll
-        for (int r = 0; r < MAXE; r++) {
-            double o = __shfl_sync(0xffffffffu, x[r], src & 31);
-            if (take) x[r] += o;
-        }
-    }
-    // ---- levels 5..log2(T)-1: warps
-#pragma unroll
-    for (int m = 0; (1 << m) < W; m++) {
-        if (lane == 31) {
-#pragma unroll
-            for (int r = 0; r < MAXE; r++) s_wt[warp][r] = x[r];
-        }
-        __syncthreads();
-        if ((warp >> m) & 1) {
-            const int sw = ((warp >> m) << m) - 1;
-#pragma unroll
-            for (int r = 0; r < MAXE; r++) x[r] += s_wt[sw][r];
-        }
-        __syncthreads();
-    }
-    // ---- levels >= log2(T): rows
-    if (E > 1) {
-        if (tid == T - 1) {
-#pragma unroll
-            for (int r = 0; r < MAXE; r++) s_rt[r] = x[r];
-        }
-        __syncthreads();
-        double rt[MAXE];
-#pragma unroll
-        for (int r = 0; r < MAXE; r++) rt[r] = s_rt[r];
+        store4(g.vcost + ti.base + i0, n - i0, vec, v);
+        x[p][1] += x[p][0];
+        x[p][3] += x[p][2];
+        x[p][2] += x[p][1];
+        x[p][3] += x[p][1];
 #pragma unroll
         for (int m = 0; m < 5; m++) {
-            if ((1 << m) >= MAXE) break;
+            const double o = __shfl_sync(kFull, x[p][3], (((lane >> m) << m) - 1) & 31);
+            if ((lane >> m) & 1)
 #pragma unroll
-            for (int r = 0; r < MAXE; r++) {
-                if ((r >> m) & 1) {
-                    const int sr = ((r >> m) << m) - 1;
-                    x[r] += rt[sr];
-                    rt[r] += rt[sr];
-                }
+                for (int j = 0; j < 4; j++) x[p][j] += o;
+        }
+    }
+    if constexpr (P > 1) {
+        const double o = __shfl_sync(kFull, x[0][3], 31);
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[1][j] += o;
+    }
+    if constexpr (W > 1) {
+        if (lane == 31) s_total[warp] = x[P - 1][3];
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; (1 << m) < W; m++) {
+            if ((warp >> m) & 1) {
+                const int last = ((warp >> m) << m) - 1;  // the 2^m warps up to it, added up as a tree
+                double o[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) o[k] = k < 1 << m ? s_total[last - k] : 0.0;
+#pragma unroll
+                for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2 * h)
+                        if (k + h < 1 << m) o[k] += o[k + h];
+#pragma unroll
+                for (int p = 0; p < P; p++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) x[p][j] += o[0];
             }
         }
     }
 #pragma unroll
-    for (int r = 0; r < MAXE; r++) {
-        const int i = tid + r * T;
-        if (r < E && i < n) g.presum[ti.base + i] = x[r];
+    for (int p = 0; p < P; p++) {
+        const int i0 = warp * P * kPassCells + p * kPassCells + 4 * lane;
+        store_sums(g.presum + ti.base + i0, n - i0, vec, x[p], s_stage[warp], lane);
     }
 }
 
-// Copies n floats of a track's capacity (when `a` is non-null) and demand into
+// whether a track's arrays can be read and written 16 (sums: 32) bytes at a time
+__device__ __forceinline__ bool track_vec(const GridDev &g, const TrackInfo &ti) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(g.cap + ti.base) | reinterpret_cast<uintptr_t>(g.demand + ti.base) |
+                        reinterpret_cast<uintptr_t>(g.vcost + ti.base);
+    return ((a | reinterpret_cast<uintptr_t>(g.presum + ti.base) >> 1) & 15) == 0;
+}
+
+template <int W, int P>
+__global__ void __launch_bounds__(32 * W, 28 / W) cost_refresh_kernel(GridDev g, int only_dirty) {
+    chain_begin();
+    const int tr = blockIdx.x;
+    if (only_dirty) {
+        if (!g.dirty_cost[tr]) return;
+    }
+    const TrackInfo ti = decode_track(g, tr);
+    const bool vec = track_vec(g, ti);
+    const int n = ti.len, lane = threadIdx.x & 31, first = (threadIdx.x >> 5) * P * kPassCells;
+    const float *cap = g.cap + ti.base, *dem = g.demand + ti.base;
+    TrackCells<P> t;
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        const int i0 = first + p * kPassCells + 4 * lane;
+        load4(cap + i0, n - i0, vec, t.c[p]);
+        load4(dem + i0, n - i0, vec, t.d[p]);
+    }
+    const bool before = lane == 0 && first > 0 && first <= n;
+    const float pc = before ? cap[first - 1] : 0.f, pd = before ? dem[first - 1] : 0.f;
+    refresh_track<W, P>(g, ti, t, pc, pd, vec, 2);
+    if (only_dirty) {
+        if (W == 1) __syncwarp();  // every lane has seen the flag (warps: refresh_track's barrier)
+        if (threadIdx.x == 0) g.dirty_cost[tr] = 0;
+    }
+}
+
+// Copies n floats of a track's capacity and demand into
 // shared memory in one loop, so that the loads of both arrays are in flight
 // together: 16 bytes per load where the track starts on a 16-byte boundary
 // (every track of a grid whose X*Y and track lengths are multiples of 4), else
@@ -204,41 +286,19 @@ __device__ __forceinline__ void stage_track(const float *a, const float *b, floa
         float4 *da4 = reinterpret_cast<float4 *>(da), *db4 = reinterpret_cast<float4 *>(db);
         for (int i = tid; i < n4; i += nthreads) {
             const float4 vb = b4[i];
-            if (a) da4[i] = a4[i];
+            da4[i] = a4[i];
             db4[i] = vb;
         }
         for (int i = (n4 << 2) + tid; i < n; i += nthreads) {
-            if (a) da[i] = a[i];
+            da[i] = a[i];
             db[i] = b[i];
         }
     } else {
         for (int i = tid; i < n; i += nthreads) {
-            if (a) da[i] = a[i];
+            da[i] = a[i];
             db[i] = b[i];
         }
     }
-}
-
-// Threads per track of the per-track kernels: five CTAs of 256 per SM (a
-// CTA of 512 or 1024 threads per track shortens each track's chain but keeps
-// fewer tracks in flight per SM, and the refresh is issue-bound: 17.2 and
-// 28.2 ms against 11.5 ms per route of the 800k-net design).
-#define IGR_TRACK_BOUNDS(T) __launch_bounds__(T, 5)
-
-template <int T, int MAXE>
-__global__ void IGR_TRACK_BOUNDS(T) cost_refresh_kernel(GridDev g, int only_dirty) {
-    chain_begin();
-    const int tr = blockIdx.x;
-    if (only_dirty) {
-        if (!g.dirty_cost[tr]) return;
-    }
-    const TrackInfo ti = decode_track(g, tr);
-    extern __shared__ __align__(16) float s_track[];  // capacity, demand, unit-step cost: MAXE * T each
-    float *s_cap = s_track, *s_dem = s_track + MAXE * T, *s_of1 = s_track + 2 * MAXE * T;
-    stage_track(g.cap + ti.base, g.demand + ti.base, s_cap, s_dem, ti.len, threadIdx.x, T);
-    __syncthreads();
-    if (threadIdx.x == 0 && only_dirty) g.dirty_cost[tr] = 0;
-    refresh_track<T, MAXE>(g, ti, s_cap, s_dem, s_of1, 2);
 }
 
 // Tracks of more than 4096 cells (up to the reference's 15,360, main.cpp:28):
@@ -306,72 +366,104 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
 // per cell are added where this batch's wires left no stamp
 // (commit_via_demand, graph.hpp:496-543: half a unit on each track edge
 // beside the cell, a full unit at the track ends), and the costs and prefix
-// sums are rebuilt from the demand still in shared memory.  Tracks with no
-// pending commit and clean costs are skipped.  With refresh = 0 the costs are
-// only marked dirty.
-template <int T, int MAXE>
-__global__ void IGR_TRACK_BOUNDS(T) commit_refresh_kernel(GridDev g, int *vcnt, int stamp, int refresh) {
-    extern __shared__ __align__(16) float s_track[];  // capacity, demand, unit-step cost: MAXE * T each
-    float *s_cap = s_track, *s_dem = s_track + MAXE * T, *s_of1 = s_track + 2 * MAXE * T;
-    __shared__ int s_w[T / 32];
-    __shared__ int s_carry;
-    __shared__ long long s_wl[T / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// sums are rebuilt from the demand in registers.  Tracks with no pending commit
+// and clean costs are skipped.  With refresh = 0 the costs are only marked dirty.
+template <int W, int P>
+__global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev g, int *vcnt, int stamp, int refresh) {
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ int s_sum[W];
+    __shared__ float s_first[W + 1], s_last[W];
+    __shared__ long long s_wl[W];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = warp * P * kPassCells;
     const int tr = blockIdx.x;
     const bool commit = g.dirty_commit[tr] != 0;
     if (!commit && !(refresh && g.dirty_cost[tr])) return;
     const TrackInfo ti = decode_track(g, tr);
     const int n = ti.len;
-    stage_track(refresh ? g.cap + ti.base : nullptr, g.demand + ti.base, s_cap, s_dem, n, tid, T);
+    const bool vec = track_vec(g, ti);
+    float *dem = g.demand + ti.base;
+    const float *cap = g.cap + ti.base;
+    TrackCells<P> t;
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+        const int i0 = first + p * kPassCells + 4 * lane;
+        if (refresh) load4(cap + i0, n - i0, vec, t.c[p]);
+        load4(dem + i0, n - i0, vec, t.d[p]);
+    }
+    float pd = lane == 0 && first > 0 && first <= n ? dem[first - 1] : 0.f;
+    const float pc = refresh && lane == 0 && first > 0 && first <= n ? cap[first - 1] : 0.f;
     if (commit) {
         const int *elen = ti.dir ? g.ylen : g.xlen;
-        if (tid == 0) s_carry = 0;
-        __syncthreads();
-        long long wl = 0;
-        for (int r0 = 0; r0 < n; r0 += T) {
-            const int i = r0 + tid;
-            int v = 0;
-            if (i < n) {
-                v = g.pre[ti.base + i];
-                if (v != 0) g.pre[ti.base + i] = 0;
-            }
-            const int inc = warp_incl_scan(v, lane);
-            if (lane == 31) s_w[warp] = inc;
-            __syncthreads();
-            int wpre = 0;
-            for (int w = 0; w < warp; w++) wpre += s_w[w];
-            const int cnt = s_carry + wpre + inc;  // inclusive prefix at i
-            if (i < n - 1 && cnt > 0) {
-                s_dem[i] += (float)cnt;
-                g.stamp[ti.base + i] = stamp;
-                wl += (long long)cnt * elen[i];
-            }
-            __syncthreads();
-            if (tid == T - 1) s_carry = cnt;
-            __syncthreads();
-        }
-        // vias, after every wire stamp of the track is in place
-        for (int i = tid; i < n; i += T) {
-            const int c = vcnt[ti.base + i];
-            if (c == 0) continue;
-            vcnt[ti.base + i] = 0;
-            if (g.stamp[ti.base + i] >= stamp) continue;
-            if (i == 0) atomicAdd(&s_dem[0], (float)c);
-            else if (i == n - 1) atomicAdd(&s_dem[n - 2], (float)c);
-            else {
-                atomicAdd(&s_dem[i - 1], 0.5f * (float)c);
-                atomicAdd(&s_dem[i], 0.5f * (float)c);
-            }
-        }
+        int *pre = g.pre + ti.base, *vc = vcnt + ti.base, *stp = g.stamp + ti.base;
+        const bool pvec = ((reinterpret_cast<uintptr_t>(pre) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
+        int cnt[P][4], via[P][4], run = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) wl += __shfl_down_sync(0xffffffffu, wl, o);
+        for (int p = 0; p < P; p++) {
+            const int i0 = first + p * kPassCells + 4 * lane;
+            load4(pre + i0, n - i0, pvec, cnt[p]);
+            load4(vc + i0, n - i0, pvec, via[p]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (cnt[p][j] != 0) pre[i0 + j] = 0;
+                if (via[p][j] != 0) vc[i0 + j] = 0;
+                if (j) cnt[p][j] += cnt[p][j - 1];
+            }
+            const int sum = cnt[p][3], inc = warp_incl_scan(sum, lane);
+#pragma unroll
+            for (int j = 0; j < 4; j++) cnt[p][j] += run + inc - sum;
+            run += __shfl_sync(kFull, inc, 31);
+        }
+        if (lane == 0) s_sum[warp] = run;
+        __syncthreads();
+        int base = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) base += w < warp ? s_sum[w] : 0;
+        // wires: demand, stamps, wirelength; then the vias of cells without this batch's stamp
+        long long wl = 0;
+        float own[P][4], prev[P][4];  // a via's part of its own edge and of the one before
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int i = first + p * kPassCells + 4 * lane + j, k = cnt[p][j] + base;
+                const bool wire = i < n - 1 && k > 0;
+                if (wire) {
+                    t.d[p][j] += (float)k;
+                    stp[i] = stamp;
+                    wl += (long long)k * elen[i];
+                }
+                const float c = (float)via[p][j];
+                const bool add = via[p][j] != 0 && !wire && stp[i] < stamp;
+                own[p][j] = !add || i == n - 1 ? 0.f : i == 0 ? c : 0.5f * c;
+                prev[p][j] = !add || i == 0 ? 0.f : i == n - 1 ? c : 0.5f * c;
+            }
+        }
+        if (lane == 0) s_first[warp] = prev[0][0];
+        if (tid == 0) s_first[W] = 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) wl += __shfl_down_sync(kFull, wl, o);
         if (lane == 0) s_wl[warp] = wl;
         __syncthreads();
-        for (int i = tid; i < n; i += T) g.demand[ti.base + i] = s_dem[i];
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            float next = __shfl_down_sync(kFull, prev[p][0], 1);
+            const float other = p == P - 1 ? s_first[warp + 1] : __shfl_sync(kFull, prev[P - 1][0], 0);
+            if (lane == 31) next = other;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                t.d[p][j] += own[p][j];
+                t.d[p][j] += j < 3 ? prev[p][j + 1] : next;
+            }
+            const int i0 = first + p * kPassCells + 4 * lane;
+            store4(dem + i0, n - i0, vec, t.d[p]);
+        }
+        if (lane == 31) s_last[warp] = t.d[P - 1][3];
+        __syncthreads();
+        if (lane == 0 && warp > 0) pd = s_last[warp - 1];
         if (tid == 0) {
-            long long t = 0;
-            for (int w = 0; w < T / 32; w++) t += s_wl[w];
-            if (t) atomicAdd(&g.stats[0], (unsigned long long)t);
+            long long sum = 0;
+            for (int w = 0; w < W; w++) sum += s_wl[w];
+            if (sum) atomicAdd(&g.stats[0], (unsigned long long)sum);
             atomicAdd(&g.stats[3], (unsigned long long)n);  // committed cells, for the roofline
             g.dirty_commit[tr] = 0;
             g.dirty_cost[tr] = refresh ? 0 : 1;
@@ -380,7 +472,7 @@ __global__ void IGR_TRACK_BOUNDS(T) commit_refresh_kernel(GridDev g, int *vcnt, 
         __syncthreads();
         if (tid == 0) g.dirty_cost[tr] = 0;
     }
-    if (refresh) refresh_track<T, MAXE>(g, ti, s_cap, s_dem, s_of1, 4);
+    if (refresh) refresh_track<W, P>(g, ti, t, pc, pd, vec, 4);
 }
 
 template <typename T>
@@ -407,49 +499,39 @@ __global__ void track_to_ref_kernel(GridDev g, const T *trk, T *ref) {
 
 }  // namespace
 
-// dynamic shared memory of a track kernel: capacity, demand and unit-step
-// cost of T * E cells
-template <int T, int E>
-constexpr size_t track_smem() { return (size_t)3 * T * E * sizeof(float); }
-
 // One CTA per track: the hardware block scheduler hands the dirty tracks to
 // the SMs as they free up, and a CTA that finds its track clean exits at once
 // (a resident grid striding over the tracks balanced the uneven dirty tracks
 // worse: 11.9 -> 15.8 ms per route of the 800k-net design; a resident grid
 // over a list of the dirty tracks made by a one-CTA pass saved nothing).
-template <int T, int E>
-static void cost_refresh_e(const GridDev &g, int od, cudaStream_t s) {
-    constexpr size_t smem = track_smem<T, E>();
-    kernel_setup((const void *)cost_refresh_kernel<T, E>, T, smem);
-    launch_chained(cost_refresh_kernel<T, E>, dim3(g.ntracks), dim3(T), smem, s, g, od);
-}
-
-template <int T, int E>
-static void commit_refresh_e(const GridDev &g, int *vcnt, int stamp, int rf, cudaStream_t s) {
-    constexpr size_t smem = track_smem<T, E>();
-    kernel_setup((const void *)commit_refresh_kernel<T, E>, T, smem);
-    commit_refresh_kernel<T, E><<<g.ntracks, T, smem, s>>>(g, vcnt, stamp, rf);
-}
-
-// Calls f(E) with E = the rows per thread of a 256-thread CTA for tracks of
-// maxlen <= kMaxFusedTrackCells cells, exactly ceil(maxlen / 256): rows that
-// hold no cell of any track would still be scanned.
-template <int E, class F>
-static void with_rows(int e, F &&f) {
-    if constexpr (E * kTrackThreads >= kMaxFusedTrackCells) {
-        f(std::integral_constant<int, E>());
+//
+// Calls f(W, P) with W warps of P passes per track for tracks of maxlen <=
+// kMaxFusedTrackCells cells.  One
+// pass up to 1024 cells, where the shorter chain counts (a track of 61 cells: 6.8 us
+// in place of 9.7), two above, where 13 warps of one pass took 179 us for 153.
+template <int P, int W, class F>
+static void with_warps(int w, F &&f) {
+    if constexpr (W * P * kPassCells >= (P == 1 ? kOnePassCells : kMaxFusedTrackCells)) {
+        f(std::integral_constant<int, W>(), std::integral_constant<int, P>());
     } else {
-        if (e <= E) f(std::integral_constant<int, E>());
-        else with_rows<E + 1>(e, f);
+        if (w <= W) f(std::integral_constant<int, W>(), std::integral_constant<int, P>());
+        else with_warps<P, W + 1>(w, f);
     }
+}
+template <class F>
+static void with_track_shape(int maxlen, F &&f) {
+    if (maxlen <= kOnePassCells) with_warps<1, 1>((maxlen + kPassCells - 1) / kPassCells, f);
+    else with_warps<2, kOnePassCells / (2 * kPassCells) + 1>((maxlen + 2 * kPassCells - 1) / (2 * kPassCells), f);
 }
 
 void launch_cost_refresh(const GridDev &g, bool only_dirty, cudaStream_t s) {
     const int maxlen = g.X > g.Y ? g.X : g.Y;
     const int od = only_dirty ? 1 : 0;
     if (maxlen <= kMaxFusedTrackCells) {
-        with_rows<1>((maxlen + kTrackThreads - 1) / kTrackThreads,
-                     [&](auto ec) { cost_refresh_e<kTrackThreads, decltype(ec)::value>(g, od, s); });
+        with_track_shape(maxlen, [&](auto wc, auto pc) {
+            constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
+            launch_chained(cost_refresh_kernel<W, P>, dim3(g.ntracks), dim3(32 * W), 0, s, g, od);
+        });
     } else {
         const size_t smem = (size_t)kMaxTrackCells * 8;
         kernel_setup((const void *)cost_refresh_long_kernel, kLongThreads, smem);
@@ -461,8 +543,10 @@ void launch_commit_refresh(const GridDev &g, int *vcnt, int stamp, bool refresh,
     const int maxlen = g.X > g.Y ? g.X : g.Y;
     if (maxlen > kMaxFusedTrackCells) throw Error(ERR_STATE, "fused batch commit on tracks longer than 4096 cells");
     const int rf = refresh ? 1 : 0;
-    with_rows<1>((maxlen + kTrackThreads - 1) / kTrackThreads,
-                 [&](auto ec) { commit_refresh_e<kTrackThreads, decltype(ec)::value>(g, vcnt, stamp, rf, s); });
+    with_track_shape(maxlen, [&](auto wc, auto pc) {
+        constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
+        commit_refresh_kernel<W, P><<<g.ntracks, 32 * W, 0, s>>>(g, vcnt, stamp, rf);
+    });
 }
 
 static int grid_for(int64_t n) {

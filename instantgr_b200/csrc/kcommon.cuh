@@ -78,6 +78,36 @@ __device__ __forceinline__ TrackInfo decode_track(const GridDev &g, int tr) {
     return ti;
 }
 
+// Four consecutive entries of a track from p on, `left` of which exist (the rest
+// read as 0); vec: p is 16-byte aligned.
+__device__ __forceinline__ void load4(const float *p, int left, bool vec, float (&v)[4]) {
+    if (vec && left >= 4) {
+        const float4 t = *reinterpret_cast<const float4 *>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = j < left ? p[j] : 0.f;
+    }
+}
+__device__ __forceinline__ void load4(const int *p, int left, bool vec, int (&v)[4]) {
+    if (vec && left >= 4) {
+        const int4 t = *reinterpret_cast<const int4 *>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = j < left ? p[j] : 0;
+    }
+}
+__device__ __forceinline__ void store4(float *p, int left, bool vec, const float (&v)[4]) {
+    if (vec && left >= 4) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (j < left) p[j] = v[j];
+    }
+}
+
 // of_cost_scaled (graph.hpp:23-27) with of_cost_scale = 1
 __device__ __forceinline__ double of_cost(float capacity, float demand) {
     const double scale = 1.0;

@@ -44,6 +44,28 @@ def test_cost_refresh_matches_oracle(gp):
     np.testing.assert_allclose(p, op, rtol=RTOL, atol=1e-9)
 
 
+@pytest.mark.parametrize("X,Y,via", [(2, 127, 2.0), (128, 129, 1.3), (131, 1024, 2.0), (9, 1025, 0.7), (1281, 6, 2.0),
+                                     (4096, 3, 1.3), (4097, 2, 2.0)])
+def test_cost_refresh_at_track_edges(X, Y, via):
+    """Tracks around the cells of a warp and a pass, aligned and not, via costs
+    with and without a float value; capacities without, far above and far below
+    the demand, where the overflow costs are 0, denormal, and above their cap."""
+    g = cases.grid_case(X + Y, X=X, Y=Y, dir0=X & 1, unit_via=via, unit_wire=0.3)
+    rng = np.random.default_rng(X * Y)
+    cap, dem = g["cap"].copy().ravel(), g["demand"].copy().ravel()
+    pick = rng.integers(0, 12, cap.size)
+    cap[pick == 0] = 0
+    cap[pick == 1] = rng.integers(150, 400, int((pick == 1).sum()))
+    dem[pick == 2] = rng.integers(100, 400, int((pick == 2).sum()))
+    g["cap"], g["demand"] = cap.reshape(g["cap"].shape), dem.reshape(g["demand"].shape)
+    c = ctx_for(g)
+    c.cost_refresh()
+    v, p = c.costs()
+    _, ov, op = Oracle(g).cost_refresh(g["demand"])
+    np.testing.assert_allclose(v, ov, rtol=RTOL, atol=0)
+    np.testing.assert_allclose(p, op, rtol=RTOL, atol=1e-9)
+
+
 def test_dirty_refresh_equals_full_refresh():
     g = cases.grid_case(5, X=120, Y=90, dir0=0)
     c = ctx_for(g)
