@@ -61,17 +61,34 @@ constexpr int kBuf = 4096;                     // staged list entries per block
 // group and phase at most)
 constexpr int kBlockRounds = 2 * kGroups;
 
-// flags (ints): [0..1] lost counts, [2] batches, [4..5] barrier counter, [6] error,
-// [8] rounds run, [9..10] candidate counts (both by round parity), [11..12] nets
-// left after a batch (by batch parity), [13] cells to recompute.  A counter is
-// zeroed one phase before it is used and was last read two barriers earlier.
-enum : int { F_LOST = 0, F_NB = 2, F_BAR = 4, F_ERR = 6, F_ROUNDS = 8, F_CAND = 9, F_LEFT = 11, F_DIRTY = 13 };
+// flags (ints): [0..1] and [14..15] lost counts (by round parity, of even and odd
+// batches), [2] batches, [4..5] barrier counter, [6] error, [8] rounds run, [9..10]
+// candidate counts (by round parity), [11..12] nets left after a batch (by batch
+// parity), [13] cells to recompute.  A counter is zeroed a barrier before it is used
+// and a barrier after it was last read.
+__device__ __forceinline__ int lost_counts(int batch) { return batch & 1 ? 14 : 0; }
+enum : int { F_NB = 2, F_BAR = 4, F_ERR = 6, F_ROUNDS = 8, F_CAND = 9, F_LEFT = 11, F_DIRTY = 13 };
 
 constexpr int kMaxRounds = 30;
-constexpr int kMember = 1 << 30;
-// map value of net k's claim in an epoch (the round, unless ranks leave too few
-// bits: then the other claims are cleared from time to time)
-__device__ __forceinline__ int claim_value(const ColorDev &c, int epoch, int k) { return epoch << c.rank_bits | k; }
+// Lists that take the groups of the grid at most this many steps are listed and
+// claim in one phase; longer ones are listed by a thread per net first, since the
+// claims of a step would wait for its nets' batches to be read.
+constexpr int kLeftSteps = 4;
+// A map value, from the top bit down: generation of the batch, member, epoch, rank.
+// The epoch is the round, unless ranks leave it too few bits: then the claims that
+// are not members' are cleared from time to time.  A claim of a later generation
+// is above everything of the ones before, so the map is cleared only when the
+// generations run out, and the nets that a batch left claim for the next one while
+// they are listed.
+struct Values {
+    int base, member;  // of the batch's generation: least value, least value of a member
+    int bits;          // of the rank
+    __device__ __forceinline__ int epoch(int e) const { return base + (e << bits); }  // | rank: a claim
+};
+__device__ __forceinline__ Values batch_values(const ColorDev &c, int gen) {
+    const int base = gen << (c.rank_bits + c.epoch_bits + 1);
+    return {base, base + (1 << (c.rank_bits + c.epoch_bits)), c.rank_bits};
+}
 
 // memory operations of this thread, summed into c.ops at the end (roofline
 // accounting): claimed cells, points checked for commit, points checked for
@@ -166,20 +183,51 @@ __device__ __forceinline__ void claim_cells(const ColorDev &c, int4 h, int gl, i
     }
 }
 template <int G>
-__device__ __forceinline__ void claim_nets(const ColorDev &c, const int *list, int n, int blk, int nblk, Ops &ops) {
+__device__ __forceinline__ void claim_nets(const ColorDev &c, const int *list, int n, int value, int blk, int nblk,
+                                           Ops &ops) {
     constexpr int kPer = kThreads / G;
     const int gl = threadIdx.x % G;
     for (int idx = blk * kPer + threadIdx.x / G; idx < n; idx += nblk * kPer) {
         const int k = list[idx];
         const int4 h = c.hdr[k];
         if (gl == 0) ops.claims += h.y - h.x;
-        claim_cells<G>(c, h, gl, claim_value(c, 0, k));
+        claim_cells<G>(c, h, gl, value | k);
     }
 }
 // round 0 of a batch
-__device__ __forceinline__ void claim_phase(const ColorDev &c, const int *list, int n, int blk, int nblk, Ops &ops) {
-    by_length(n, nblk, [&] { claim_nets<kG>(c, list, n, blk, nblk, ops); },
-              [&] { claim_nets<32>(c, list, n, blk, nblk, ops); });
+__device__ __forceinline__ void claim_phase(const ColorDev &c, const int *list, int n, int value, int blk, int nblk,
+                                            Ops &ops) {
+    by_length(n, nblk, [&] { claim_nets<kG>(c, list, n, value, blk, nblk, ops); },
+              [&] { claim_nets<32>(c, list, n, value, blk, nblk, ops); });
+}
+
+// The nets of `list` still without a batch go to `left` and claim for round 0 of
+// the next batch.
+template <int G>
+__device__ __forceinline__ void left_nets(const ColorDev &c, Stage &st, const int *list, int n, int *left, int *left_cnt,
+                                          int value, int blk, int nblk, Ops &ops) {
+    constexpr int kPer = kThreads / G;
+    const int lane = threadIdx.x & 31, gl = lane % G;
+    int it = 0;
+    for (int b0 = blk * kPer; b0 < n; b0 += nblk * kPer, it++) {
+        const int idx = b0 + threadIdx.x / G;
+        const int k = idx < n ? list[idx] : -1;
+        const bool stays = k >= 0 && __ldcg(c.batch + k) == -1;
+        if (k >= 0 && gl == 0) ops.scans++;
+        if (stays) {
+            const int4 h = c.hdr[k];
+            if (gl == 0) ops.claims += h.y - h.x;
+            claim_cells<G>(c, h, gl, value | k);
+        }
+        stage(st, stays && gl == 0, k, lane);
+        if ((it + 1) % (kBuf / kPer) == 0) flush(st, left, left_cnt);
+    }
+    flush(st, left, left_cnt);
+}
+__device__ __forceinline__ void left_phase(const ColorDev &c, Stage &st, const int *list, int n, int *left,
+                                           int *left_cnt, int value, int blk, int nblk, Ops &ops) {
+    by_length(n, nblk, [&] { left_nets<kG>(c, st, list, n, left, left_cnt, value, blk, nblk, ops); },
+              [&] { left_nets<32>(c, st, list, n, left, left_cnt, value, blk, nblk, ops); });
 }
 
 // Candidates owning all their points join batch `cur` and mark the cells they
@@ -187,8 +235,8 @@ __device__ __forceinline__ void claim_phase(const ColorDev &c, const int *list, 
 // this and the next phase 1.1 times slower, stopping at the first foreign point,
 // G points at a time, 1.4 times: fewer reads, but a longer chain of them.)  Block-uniform loop (staging and flushes).
 template <int G>
-__device__ __forceinline__ void commit_nets(const ColorDev &c, Stage &st, const int *list, int n, int epoch, int cur,
-                                            int *lost_cnt, int blk, int nblk, Ops &ops) {
+__device__ __forceinline__ void commit_nets(const ColorDev &c, Stage &st, const int *list, int n, const Values &vs,
+                                            int epoch, int cur, int *lost_cnt, int blk, int nblk, Ops &ops) {
     constexpr int kPer = kThreads / G;
     const int lane = threadIdx.x & 31, grp = lane / G, gl = lane % G;
     int it = 0;
@@ -196,7 +244,7 @@ __device__ __forceinline__ void commit_nets(const ColorDev &c, Stage &st, const 
         const int idx = b0 + threadIdx.x / G;
         const bool valid = idx < n;
         const int k = valid ? list[idx] : -1;
-        const int v = claim_value(c, epoch, k);
+        const int v = vs.epoch(epoch) | k, own = v + (vs.member - vs.base);
         int4 h = make_int4(0, 0, 0, 0);
         bool ok = true;
         if (valid) {
@@ -224,7 +272,7 @@ __device__ __forceinline__ void commit_nets(const ColorDev &c, Stage &st, const 
                 for (int u = 0; u < 4; u++) ow[u] = cl[u] >= 0 ? owner(c, cl[u]) : -1;
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    if (ow[u] == v) c.map[cl[u]] = v | kMember;
+                    if (ow[u] == v) c.map[cl[u]] = own;
             }
         }
         stage(st, valid && bad != 0 && gl == 0, k, lane);
@@ -232,17 +280,17 @@ __device__ __forceinline__ void commit_nets(const ColorDev &c, Stage &st, const 
     }
     flush(st, c.lost, lost_cnt);
 }
-__device__ __forceinline__ void commit_phase(const ColorDev &c, Stage &st, const int *list, int n, int epoch, int cur,
-                                             int *lost_cnt, int blk, int nblk, Ops &ops) {
-    by_length(n, nblk, [&] { commit_nets<kG>(c, st, list, n, epoch, cur, lost_cnt, blk, nblk, ops); },
-              [&] { commit_nets<32>(c, st, list, n, epoch, cur, lost_cnt, blk, nblk, ops); });
+__device__ __forceinline__ void commit_phase(const ColorDev &c, Stage &st, const int *list, int n, const Values &vs,
+                                             int epoch, int cur, int *lost_cnt, int blk, int nblk, Ops &ops) {
+    by_length(n, nblk, [&] { commit_nets<kG>(c, st, list, n, vs, epoch, cur, lost_cnt, blk, nblk, ops); },
+              [&] { commit_nets<32>(c, st, list, n, vs, epoch, cur, lost_cnt, blk, nblk, ops); });
 }
 
 // Lost nets with a point owned by a member are blocked for this batch; the
 // others stay candidates and claim their cells for the next round, `epoch`.
 template <int G>
-__device__ __forceinline__ void next_nets(const ColorDev &c, Stage &st, int n, int epoch, int *cand_cnt, int blk,
-                                          int nblk, Ops &ops) {
+__device__ __forceinline__ void next_nets(const ColorDev &c, Stage &st, int n, const Values &vs, int epoch,
+                                          int *cand_cnt, int blk, int nblk, Ops &ops) {
     constexpr int kPer = kThreads / G;
     const int lane = threadIdx.x & 31, grp = lane / G, gl = lane % G;
     int it = 0;
@@ -260,28 +308,29 @@ __device__ __forceinline__ void next_nets(const ColorDev &c, Stage &st, int n, i
                 const int p1 = i + G < h.w ? __ldg(c.pts + i + G) : -1;
                 const int o0 = owner(c, p0);
                 const int o1 = p1 >= 0 ? owner(c, p1) : -1;
-                hit |= (o0 >= kMember) | (o1 >= kMember);
+                hit |= (o0 >= vs.member) | (o1 >= vs.member);
             }
         }
         const bool blocked = ((__ballot_sync(0xffffffffu, hit) >> (grp * G)) & (0xffffffffu >> (32 - G))) != 0;
         if (valid && !blocked) {
             if (gl == 0) ops.claims += h.y - h.x;
-            claim_cells<G>(c, h, gl, claim_value(c, epoch, k));
+            claim_cells<G>(c, h, gl, vs.epoch(epoch) | k);
         }
         stage(st, valid && !blocked && gl == 0, k, lane);
         if ((it + 1) % (kBuf / kPer) == 0) flush(st, c.cand, cand_cnt);
     }
     flush(st, c.cand, cand_cnt);
 }
-__device__ __forceinline__ void next_phase(const ColorDev &c, Stage &st, int n, int epoch, int *cand_cnt, int blk,
-                                           int nblk, Ops &ops) {
-    by_length(n, nblk, [&] { next_nets<kG>(c, st, n, epoch, cand_cnt, blk, nblk, ops); },
-              [&] { next_nets<32>(c, st, n, epoch, cand_cnt, blk, nblk, ops); });
+__device__ __forceinline__ void next_phase(const ColorDev &c, Stage &st, int n, const Values &vs, int epoch,
+                                           int *cand_cnt, int blk, int nblk, Ops &ops) {
+    by_length(n, nblk, [&] { next_nets<kG>(c, st, n, vs, epoch, cand_cnt, blk, nblk, ops); },
+              [&] { next_nets<32>(c, st, n, vs, epoch, cand_cnt, blk, nblk, ops); });
 }
 
 // Rounds `round`.. of batch `cur` in this block alone, over the nc candidates
 // in c.cand, which have claimed in that round.  Every thread of the block calls it.
-__device__ void block_rounds(const ColorDev &c, Stage &st, int round, int nc, int cur, int *rounds_ctr, Ops &ops) {
+__device__ void block_rounds(const ColorDev &c, Stage &st, const Values &vs, int round, int nc, int cur,
+                             int *rounds_ctr, Ops &ops) {
     __shared__ int s_lost, s_cand;
     while (true) {
         if (threadIdx.x == 0) {
@@ -290,11 +339,11 @@ __device__ void block_rounds(const ColorDev &c, Stage &st, int round, int nc, in
             (*rounds_ctr)++;
         }
         __syncthreads();
-        commit_phase(c, st, c.cand, nc, round, cur, &s_lost, 0, 1, ops);
+        commit_phase(c, st, c.cand, nc, vs, round, cur, &s_lost, 0, 1, ops);
         const int nl = s_lost;  // flush ends with a block barrier
         if (nl == nc || round + 1 >= kMaxRounds) break;
         round++;
-        next_phase(c, st, nl, round, &s_cand, 0, 1, ops);
+        next_phase(c, st, nl, vs, round, &s_cand, 0, 1, ops);
         nc = s_cand;
         __syncthreads();  // every thread has read the counters before they are reset
         if (nc == 0) break;
@@ -384,60 +433,72 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
         }
         if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
     }
-    int na = c.n;
+    int na = c.n, gen = 0;
+    const int gens = inc ? 1 : 1 << (30 - c.rank_bits - c.epoch_bits);
+    bool claimed = false;  // the nets without a batch have claimed for round 0
     for (int cur = 0; cur < max_batches; cur++) {
+        const Values vs = batch_values(c, gen);
+        const int f_lost = lost_counts(cur);
         const int *cand = act;  // round 0: every net without a batch
         int nc = na, epoch = 0;
         // with the round-0 map kept up to date, round 0 of a later batch starts
         // from it (its counters were reset before the last barrier)
-        const bool kept = inc && cur > 0;
-        if (!kept) {
-            if (tid == 0) flags[F_LOST] = 0;
-            claim_phase(c, cand, nc, blockIdx.x, gridDim.x, ops);
+        if (!claimed && !(inc && cur > 0)) {
+            claim_phase(c, cand, nc, vs.base, blockIdx.x, gridDim.x, ops);
             if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
-            if (tid == 0) flags[F_LEFT + ((cur + 1) & 1)] = 0;
         }
         if (inc && cur == 0)  // the first round-0 map, whether or not its owners have joined yet
             for (int i = tid; i < XY; i += nth) {
                 const int v = __ldcg(c.map + i);
-                c.snap[i] = v >= 0 ? v & ~kMember : v;
+                c.snap[i] = v >= vs.member ? v - vs.member : v;
             }
         for (int round = 0;; epoch++) {
             if (tid == 0) {
                 flags[F_ROUNDS]++;
                 flags[F_CAND + ((round + 1) & 1)] = 0;
             }
-            commit_phase(c, st, cand, nc, epoch, cur, flags + F_LOST + (round & 1), blockIdx.x, gridDim.x, ops);
+            commit_phase(c, st, cand, nc, vs, epoch, cur, flags + f_lost + (round & 1), blockIdx.x, gridDim.x, ops);
             if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
-            const int nl = vflags[F_LOST + (round & 1)];
+            if (tid == 0 && round == 0) {  // the next batch's counters
+                flags[F_LEFT + ((cur + 1) & 1)] = 0;
+                flags[lost_counts(cur + 1)] = 0;
+            }
+            const int nl = vflags[f_lost + (round & 1)];
             if (nl == nc || round + 1 >= kMaxRounds) break;  // no net joined, or the last round
             round++;
-            if ((epoch + 1) >> (30 - c.rank_bits)) {  // out of epochs: clear all claims but the members'
+            if ((epoch + 1) >> c.epoch_bits) {  // out of epochs: clear all claims but the members'
                 for (int i = tid; i < XY; i += nth)
-                    if (__ldcg(c.map + i) < kMember) c.map[i] = -1;
+                    if (__ldcg(c.map + i) < vs.member) c.map[i] = -1;
                 epoch = -1;
                 if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
             }
-            if (tid == 0) flags[F_LOST + (round & 1)] = 0;
-            next_phase(c, st, nl, epoch + 1, flags + F_CAND + (round & 1), blockIdx.x, gridDim.x, ops);
+            if (tid == 0) flags[f_lost + (round & 1)] = 0;
+            next_phase(c, st, nl, vs, epoch + 1, flags + F_CAND + (round & 1), blockIdx.x, gridDim.x, ops);
             if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
             cand = c.cand;
             nc = vflags[F_CAND + (round & 1)];
             if (nc == 0) break;
             // the tail counts its rounds as epochs
-            if (nc <= kBlockRounds && epoch + 1 == round && !(kMaxRounds >> (30 - c.rank_bits))) {
-                if (blockIdx.x == 0) block_rounds(c, st, round, nc, cur, flags + F_ROUNDS, ops);
+            if (nc <= kBlockRounds && epoch + 1 == round && !(kMaxRounds >> c.epoch_bits)) {
+                if (blockIdx.x == 0) block_rounds(c, st, vs, round, nc, cur, flags + F_ROUNDS, ops);
                 if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
                 break;
             }
         }
-        // nets still without a batch stay active; the map is cleared for the
-        // next batch, or, when the round-0 map is kept, the cells whose
-        // round-0 owner joined this batch are marked for recomputation
-        if (!inc)
+        // nets still without a batch stay active and claim for the next batch; out
+        // of generations, the map is cleared instead, or, when the round-0 map is
+        // kept, the cells whose round-0 owner joined this batch are marked for
+        // recomputation
+        const bool fresh = gen + 1 < gens;
+        gen = fresh ? gen + 1 : 0;
+        claimed = fresh && na <= kLeftSteps * (int)gridDim.x * kGroups;
+        if (!inc && !fresh)
             for (int i = tid; i < XY; i += nth) c.map[i] = -1;
+        if (claimed)
+            left_phase(c, st, act, na, act2, flags + F_LEFT + (cur & 1), batch_values(c, gen).base, blockIdx.x,
+                       gridDim.x, ops);
         int it = 0;
-        for (int b0 = blockIdx.x * kThreads; b0 < na; b0 += nth, it++) {
+        for (int b0 = blockIdx.x * kThreads; b0 < na && !claimed; b0 += nth, it++) {
             const int i = b0 + threadIdx.x;
             const int k = i < na ? act[i] : -1;
             const int bk = k >= 0 ? __ldcg(c.batch + k) : -2;
@@ -496,11 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1) coloring_kernel(ColorDev c, int m
             }
             if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
             for (int i = tid; i < XY; i += nth) c.map[i] = c.snap[i];
-            if (tid == 0) {  // counters of round 0 of the next batch
-                flags[F_DIRTY] = 0;
-                flags[F_LOST] = 0;
-                flags[F_LEFT + ((cur + 2) & 1)] = 0;
-            }
+            if (tid == 0) flags[F_DIRTY] = 0;
             if (!grid_sync(bar, err, epoch_of_bar, c.wait_ns, c.phantom)) return;
         }
     }
@@ -560,7 +617,8 @@ int run_coloring(ColorDev &c, int max_batch, cudaStream_t s) {
     if (blocks < 1) blocks = 1;
     c.wait_ns = (unsigned long long)test_hooks().wait_ns.load();
     c.phantom = (unsigned)test_hooks().barrier_phantom.load();
-    for (c.rank_bits = 25; c.rank_bits < 29 && (c.n >> c.rank_bits) != 0;) c.rank_bits++;
+    for (c.rank_bits = 1; c.rank_bits < 29 && (c.n >> c.rank_bits) != 0;) c.rank_bits++;
+    c.epoch_bits = std::min(5, 30 - c.rank_bits);
     cudaMemsetAsync(c.flags, 0, 16 * sizeof(int), s);
     cudaMemsetAsync(c.batch, 0xff, sizeof(int) * (size_t)c.n, s);
     int max_batches = c.n + 1;

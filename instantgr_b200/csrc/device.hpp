@@ -357,7 +357,7 @@ struct ColorDev {
     unsigned long long *ops = nullptr;
     int *flags = nullptr;     // [16] device flags
     int rounds = 0;           // out: colouring rounds run
-    int rank_bits = 25;       // bits of a rank in the map (set by run_coloring)
+    int rank_bits = 25, epoch_bits = 5;  // bits of a rank and of an epoch in the map (set by run_coloring)
     // optional (all or none): the round-0 map of every batch kept up to date
     // instead of re-claimed.  rev_off/rev_cnt [X*Y]: claimers of each cell in
     // rev[] (ranks; [total claims]); snap/dirty [X*Y]; part [1024]
