@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev 
     __shared__ long long s_wl[W];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = warp * P * kPassCells;
     const int tr = blockIdx.x;
+    chain_begin();
     const bool commit = g.dirty_commit[tr] != 0;
     if (!commit && !(refresh && g.dirty_cost[tr])) return;
     const TrackInfo ti = decode_track(g, tr);
@@ -545,7 +546,7 @@ void launch_commit_refresh(const GridDev &g, int *vcnt, int stamp, bool refresh,
     const int rf = refresh ? 1 : 0;
     with_track_shape(maxlen, [&](auto wc, auto pc) {
         constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
-        commit_refresh_kernel<W, P><<<g.ntracks, 32 * W, 0, s>>>(g, vcnt, stamp, rf);
+        launch_chained(commit_refresh_kernel<W, P>, dim3(g.ntracks), dim3(32 * W), 0, s, g, vcnt, stamp, rf);
     });
 }
 

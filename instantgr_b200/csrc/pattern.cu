@@ -288,6 +288,7 @@ __device__ __forceinline__ void edge_step(NetSmem<T> &sm, const LaneRole &r, int
 template <int T>
 __global__ void __launch_bounds__(128, 4) pattern_route_kernel(GridDev g, TreeBatchDev b, int stamp) {
     extern __shared__ unsigned char smem_raw[];
+    chain_begin();
     if (b.gate && (b.gate->status != 0 || b.gate->big_nodes > (unsigned long long)b.scratch_nodes)) return;
     static_assert(T * 8 + 2 * kL <= 64 + 2 * kTab && 32 % T == 0 && T >= 5, "via columns fit the work area, blocks the slots");
     NetSmem<T> &sm = reinterpret_cast<NetSmem<T> *>(smem_raw)[threadIdx.x >> 5];
@@ -664,7 +665,7 @@ void launch_pattern_route(const GridDev &g, const TreeBatchDev &b, int stamp, cu
     const size_t smem = sizeof(Smem) * kWarps;
     const KernelShape ks = kernel_setup(kernel, kThreads, smem);
     const int blocks = std::min((b.n + kWarps - 1) / kWarps, ks.sms * ks.blocks_per_sm);
-    pattern_route_kernel<kPatternNodeTile><<<blocks, kThreads, smem, s>>>(g, b, stamp);
+    launch_chained(pattern_route_kernel<kPatternNodeTile>, dim3(blocks), dim3(kThreads), smem, s, g, b, stamp);
 }
 
 }  // namespace igr
