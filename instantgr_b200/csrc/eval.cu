@@ -21,14 +21,14 @@
 // A net's lines go into shared memory as two lists, wires (layer, track, start,
 // length) and vias (place, layers, position in the net's order), and every via
 // asks each wire and each via before it which of its layers they cover: a block
-// of 32 threads per net of up to 64 lines, 128 up to 1,024, 512 up to 8,192.
-// This is quadratic in a net's lines but moves no data beyond the lines
-// themselves, where marking every wire cell in a hash set (22M inserts on the
-// 800k-net design) was bound by random accesses to memory: an
-// evaluation of that design went from 21 to 5.1 ms (with the pins kept on the
-// device and no count read back before it; kernels 13.7 -> 4.9 ms), of the
-// 130k-net design from 4.8 to 1.05.
-// Nets of more lines, where the squares would cost more, keep the hash sets
+// of 32 threads per net of up to 64 lines, 128 up to 1,024, 512 up to 8,192; the
+// latter two put the lines into buckets by track or place first (asking every line,
+// they took 0.8 and 3.2 ms on the 800k-net design, now 0.6 and 1.05).  This moves no
+// data beyond the lines themselves, where marking every wire cell in a hash set (22M
+// inserts on that design) was bound by random accesses to memory: an evaluation of it
+// went from 21 to 2.7 ms (with the pins kept on the device and no count read back
+// before it; kernels 13.7 -> 2.5 ms), of the 130k-net design from 4.8 to 0.64.
+// Nets of more lines, which do not fit shared memory, keep the hash sets
 // keyed by (net, layer, x, y): the cells their wires cover, and their via
 // locations with the first position in the net's guide order.
 #include "kcommon.cuh"
@@ -165,11 +165,26 @@ __device__ __forceinline__ void add_stacked(const EvalDev &e, int z, int x, int 
     }
 }
 
+// Nets of more than 64 lines: wires in buckets by direction and track, vias by
+// place, so that a via asks three buckets.
+constexpr int kTracks = 128, kPlaces = 256;  // buckets
+__host__ __device__ constexpr bool in_buckets(int lines) { return lines > 64; }
+__host__ __device__ constexpr size_t eval_smem(int lines) {
+    return (size_t)lines * (sizeof(uint2) + (in_buckets(lines) ? sizeof(uint16_t) : 0));
+}
+__device__ __forceinline__ int track_bucket(bool hor, unsigned fix) { return (int)(fix & (kTracks / 2 - 1)) * 2 + hor; }
+__device__ __forceinline__ int place_bucket(unsigned x, unsigned y) {
+    return kTracks + (int)((x * 37 + y) & (kPlaces - 1));
+}
+
 // One net at a time: its lines to the lists, wire counts, then the vias.
 template <int THREADS, int LINES>
 __global__ void __launch_bounds__(THREADS) eval_net_kernel(EvalDev e, const int *list, const int *count, int *queue) {
     extern __shared__ uint2 lists[];  // wires from the front, vias from the back
     __shared__ int s_nw, s_nv, s_next;
+    constexpr int kBuckets = in_buckets(LINES) ? kTracks + kPlaces : 1;
+    __shared__ int s_end[kBuckets + 1];  // bucket b: entries s_end[b] .. s_end[b + 1] of `order`
+    uint16_t *order = reinterpret_cast<uint16_t *>(lists + LINES);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned XY = (unsigned)(e.X * e.Y), Y = (unsigned)e.Y;
     const unsigned rxy = 0xffffffffu / XY, ry = 0xffffffffu / Y;
@@ -250,20 +265,57 @@ __global__ void __launch_bounds__(THREADS) eval_net_kernel(EvalDev e, const int 
             int *w = e.wire + (hor ? cell_at_file(e, z, lo, fix) : cell_at_file(e, z, fix, lo));
             for (int c = lane; c < len; c += 32) atomicAdd(w + c, 1);
         }
+        auto layer_hor = [&](unsigned z) { return (((z - 1) & 1) ^ (unsigned)e.DIR) == 0; };
+        auto wire_bucket = [&](uint2 w) { return track_bucket(layer_hor(w.x >> 16), w.x & 0xffff); };
+        auto via_bucket = [&](uint2 v) { return place_bucket(v.x >> 16, v.x & 0xffff); };
+        if constexpr (in_buckets(LINES)) {
+            for (int i = tid; i <= kBuckets; i += THREADS) s_end[i] = 0;
+            __syncthreads();
+            for (int i = tid; i < nw; i += THREADS) atomicAdd(&s_end[wire_bucket(lists[i])], 1);
+            for (int i = tid; i < nv; i += THREADS) atomicAdd(&s_end[via_bucket(lists[LINES - 1 - i])], 1);
+            __syncthreads();
+            if (warp == 0) {  // counts to ends; filling a bucket then moves its end to its start
+                int run = 0;
+                for (int b0 = 0; b0 <= kBuckets; b0 += 32) {
+                    int v = b0 + lane <= kBuckets ? s_end[b0 + lane] : 0;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int u = __shfl_up_sync(0xffffffffu, v, o);
+                        if (lane >= o) v += u;
+                    }
+                    if (b0 + lane <= kBuckets) s_end[b0 + lane] = run + v;
+                    run += __shfl_sync(0xffffffffu, v, 31);
+                }
+            }
+            __syncthreads();
+            for (int i = tid; i < nw; i += THREADS) order[atomicSub(&s_end[wire_bucket(lists[i])], 1) - 1] = (uint16_t)i;
+            for (int i = tid; i < nv; i += THREADS)
+                order[atomicSub(&s_end[via_bucket(lists[LINES - 1 - i])], 1) - 1] = (uint16_t)(LINES - 1 - i);
+            __syncthreads();
+        }
         // vias: the layers (from 1) that no wire of the net and no earlier via covers there
         for (int i = tid; i < nv; i += THREADS) {
             const uint2 me = lists[LINES - 1 - i];
             const unsigned x = me.x >> 16, y = me.x & 0xffff, t = me.y >> 16;
             unsigned left = me.y & 0xfffe;
-            for (int k = 0; k < nw; k++) {
-                const uint2 w = lists[k];
+            auto by_wire = [&](uint2 w) {
                 const unsigned z = w.x >> 16;
-                const bool hor = (((z - 1) & 1) ^ (unsigned)e.DIR) == 0;
+                const bool hor = layer_hor(z);
                 if ((w.x & 0xffff) == (hor ? y : x) && (hor ? x : y) - (w.y & 0xffff) <= w.y >> 16) left &= ~(1u << z);
-            }
-            for (int k = 0; k < nv; k++) {
-                const uint2 v = lists[LINES - 1 - k];
+            };
+            auto by_via = [&](uint2 v) {
                 if (v.x == me.x && v.y >> 16 < t) left &= ~v.y;
+            };
+            if constexpr (in_buckets(LINES)) {
+                for (int hor = 0; hor < 2; hor++) {
+                    const int b = track_bucket(hor != 0, hor ? y : x);
+                    for (int k = s_end[b]; k < s_end[b + 1]; k++) by_wire(lists[order[k]]);
+                }
+                const int b = place_bucket(x, y);
+                for (int k = s_end[b]; k < s_end[b + 1]; k++) by_via(lists[order[k]]);
+            } else {
+                for (int k = 0; k < nw; k++) by_wire(lists[k]);
+                for (int k = 0; k < nv; k++) by_via(lists[LINES - 1 - k]);
             }
             while (left) {
                 const int z = __ffs(left) - 1;
@@ -446,7 +498,7 @@ void launch_eval_nets(const EvalDev &e, int *list, int *count, cudaStream_t s) {
     eval_class_kernel<<<(e.n + 255) / 256, 256, 0, s>>>(e, list, count);
     int *queue = count + kEvalClasses;
     auto run = [&](auto kernel, int threads, int cls) {
-        const size_t smem = (size_t)lines_of(cls) * sizeof(uint2);
+        const size_t smem = eval_smem(lines_of(cls));
         const KernelShape ks = kernel_setup((const void *)kernel, threads, smem);
         kernel<<<std::min(e.n, ks.sms * ks.blocks_per_sm), threads, smem, s>>>(e, list + (size_t)cls * e.n,
                                                                               count + cls, queue + cls);
