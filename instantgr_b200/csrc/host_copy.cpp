@@ -15,6 +15,7 @@
 #include <exception>
 #include <mutex>
 #include <thread>
+#include <vector>
 
 #include "router.hpp"
 
@@ -56,12 +57,22 @@ void run_workers(int n, F &&fn) {
     if (err) std::rethrow_exception(err);
 }
 
-// a worker's page-locked chunk and the event of its last copy
+// a worker's page-locked chunk (a plain one where page-locked memory has run out:
+// copies of it are staged by the driver) and the event of its last copy
 struct Slot {
     PinnedBuf<unsigned char> buf;
+    std::vector<unsigned char> plain;
+    unsigned char *p = nullptr;
     cudaEvent_t ev = nullptr;
     Slot() {
-        buf.alloc(kChunk);
+        try {
+            buf.alloc(kChunk);
+            p = buf.p;
+        } catch (const Error &) {
+            (void)cudaGetLastError();
+            plain.resize(kChunk);
+            p = plain.data();
+        }
         cuda_check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
     }
     ~Slot() {
@@ -114,10 +125,10 @@ void copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s) {
         return;
     }
     by_chunks(bytes, 1, s, [&](Slot &slot, size_t at, size_t n) {
-        cuda_check(cudaMemcpyAsync(slot.buf.p, static_cast<const char *>(src) + at, n, cudaMemcpyDeviceToHost, s), "D2H");
+        cuda_check(cudaMemcpyAsync(slot.p, static_cast<const char *>(src) + at, n, cudaMemcpyDeviceToHost, s), "D2H");
         cuda_check(cudaEventRecord(slot.ev, s), "event");
         cuda_check(cudaEventSynchronize(slot.ev), "D2H");
-        std::memcpy(static_cast<char *>(dst) + at, slot.buf.p, n);
+        std::memcpy(static_cast<char *>(dst) + at, slot.p, n);
     });
 }
 
@@ -128,8 +139,8 @@ void copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t s) {
     }
     by_chunks(bytes, 1, s, [&](Slot &slot, size_t at, size_t n) {
         cuda_check(cudaEventSynchronize(slot.ev), "H2D");  // the slot's last copy (none yet: returns at once)
-        std::memcpy(slot.buf.p, static_cast<const char *>(src) + at, n);
-        cuda_check(cudaMemcpyAsync(static_cast<char *>(dst) + at, slot.buf.p, n, cudaMemcpyHostToDevice, s), "H2D");
+        std::memcpy(slot.p, static_cast<const char *>(src) + at, n);
+        cuda_check(cudaMemcpyAsync(static_cast<char *>(dst) + at, slot.p, n, cudaMemcpyHostToDevice, s), "H2D");
         cuda_check(cudaEventRecord(slot.ev, s), "event");
     });
 }
@@ -149,8 +160,8 @@ void copy_to_device_bf16(__nv_bfloat16 *dst, const float *src, size_t n, cudaStr
     }
     by_chunks(n, 2, s, [&](Slot &slot, size_t at, size_t m) {
         cuda_check(cudaEventSynchronize(slot.ev), "H2D");
-        convert_to_bf16(src + at, m, reinterpret_cast<__nv_bfloat16 *>(slot.buf.p));
-        cuda_check(cudaMemcpyAsync(dst + at, slot.buf.p, m * 2, cudaMemcpyHostToDevice, s), "H2D");
+        convert_to_bf16(src + at, m, reinterpret_cast<__nv_bfloat16 *>(slot.p));
+        cuda_check(cudaMemcpyAsync(dst + at, slot.p, m * 2, cudaMemcpyHostToDevice, s), "H2D");
         cuda_check(cudaEventRecord(slot.ev, s), "event");
     });
 }
