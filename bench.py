@@ -499,11 +499,11 @@ def main():
         roof["kernel_classes_from"] = "one route of a profiled twin (CUDA events around every launch), untimed"
 
         # the tensor-core kernel: the learned seed's forward convolutions
-        # (umma_gemm_kernel) over 16 tiles of 288 x 288 GCells, CUDA events
+        # (conv_kernel) over 16 tiles of 288 x 288 GCells, CUDA events
         try:
             tf = model.time_forward(tiles=16, reps=5)
             roof["tensor_core"] = dict(
-                kernel="umma_gemm_kernel (tcgen05.mma kind::f16, BF16 operands, f32 accumulators in TMEM; "
+                kernel="conv_kernel (tcgen05.mma kind::f16, BF16 operands, f32 accumulators in TMEM; "
                        "the seed network's six 3x3 convolutions as implicit GEMMs, 16 tiles of 288x288)",
                 bound="tensor", unit="TFLOP/s", achieved=round(tf["tflops"], 2), peak=pk["bf16_tflops"],
                 frac=round(tf["tflops"] / pk["bf16_tflops"], 4), peak_src=pk["src"] + " (cuBLAS bf16 burst)",
@@ -516,7 +516,7 @@ def main():
         roof["latency_bound_classes"] = {
             "coloring": "grid barriers and dependent L2 accesses; DRAM nearly idle (profiles/coloring_kernel_c1.md)",
             "pattern_dp": "issue/latency bound tree DP (profiles/pattern_route_kernel_c1_largest_batch.md)",
-            "dag_dp": "bound by the dependent levels of the largest DAGs (profiles/dag_net_kernel_c2.md)",
+            "dag_dp": "bound by the dependent levels of the largest DAGs (profiles/dag_net_kernel_c2_window.md)",
         }
         cpu = None
         rgpu = None
