@@ -3,7 +3,7 @@
 //
 // Replaces three full-grid kernels of InstantGR (update_wcost_cuda_ispd24,
 // update_vcost_ispd24, compute_presum; src/graph.hpp:40-71, :101-104,
-// :405-430).  One CTA owns one track, a warp of it 256 consecutive cells: it
+// :405-430).  A CTA owns one track (several short ones), a warp 256 consecutive cells: it
 // loads capacity and demand, evaluates the cost model for every cell, writes
 // vcost (f32), and scans the wire costs in f64 into presum.  The wire cost array
 // itself is never written: 20 bytes of DRAM traffic per cell (4+4 read, 4+8
@@ -103,6 +103,50 @@ __device__ __forceinline__ void unit_costs(float c, float d, double sc, float &o
 // and a path for cells with capacity alone took fewer instructions but 164 to 172 us.)
 constexpr int kPassCells = 128;
 constexpr int kOnePassCells = 1024;  // tracks of at most this many cells: one pass a warp
+
+// A block has the warps that a track of the longer direction needs; of the other
+// direction it takes as many tracks as fit, each with the warps it needs.  (With a
+// block per track of either, the others' warps evaluated the cost model for cells that
+// are not there: 64 x 4096 cells took 645 us a call, 2000 x 200 136, now 85 and 57;
+// 840 x 1140, where that was one of the five warps of every second layer, 92 and 87.)
+// Tracks of a block share its barriers, though they need not come to the same number
+// of them: a warp without a track, or done with it, leaves the kernel, and a barrier waits
+// for the threads still in it.
+struct TrackSplit {
+    int warps0, warps1;    // per track, of the layers along x and along y
+    int tracks0, tracks1;  // per block
+};
+// this warp's track and its number among the track's warps and the block's
+struct TrackWarp {
+    TrackInfo ti;
+    int tr, warp, slot;
+    __device__ __forceinline__ bool leader() const { return warp == 0 && (threadIdx.x & 31) == 0; }
+};
+// blocks x: of a layer, y: layer; false: no track for this warp.  MIXED: some tracks take
+// fewer warps than the block has (none does at 1600 x 1600: 170 us a call without this, 174 with it).
+template <bool MIXED>
+__device__ __forceinline__ bool own_track(const GridDev &g, const TrackSplit &sp, TrackWarp &tw) {
+    const int l = blockIdx.y, dir = layer_dir(g, l);
+    int t = blockIdx.x;
+    if constexpr (MIXED) {
+        const int warps = dir ? sp.warps1 : sp.warps0, tracks = dir ? sp.tracks1 : sp.tracks0;
+        tw.slot = tw.warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // shuffled: uniform, for the compiler
+        int group = 0;
+        for (; tw.warp >= warps; tw.warp -= warps) group++;
+        if (group >= tracks) return false;
+        t = t * tracks + group;
+    } else {
+        tw.slot = tw.warp = threadIdx.x >> 5;
+    }
+    if (t >= (dir ? g.X : g.Y)) return false;
+    tw.tr = (l >> 1) * (g.X + g.Y) + (l & 1) * (g.DIR ? g.X : g.Y) + t;
+    tw.ti.l = l;
+    tw.ti.t = t;
+    tw.ti.dir = dir;
+    tw.ti.len = dir ? g.Y : g.X;
+    tw.ti.base = (int64_t)l * g.X * g.Y + (int64_t)t * tw.ti.len;
+    return true;
+}
 template <int P>
 struct TrackCells {
     float c[P][4], d[P][4];
@@ -137,8 +181,8 @@ __device__ __forceinline__ double int_to_double(int v) {  // 2^52 + 2^31 + v, le
     return __hiloint2double(0x43300000, v ^ (int)0x80000000) - 4503601774854144.0;
 }
 
-// Cost model and Sklansky prefix sums of one track of n cells; every thread of
-// the block calls it and tallies n in g.stats[slot].  (pc, pd): capacity and demand
+// Cost model and Sklansky prefix sums of one track of n cells; every warp of
+// the track calls it and n is tallied in g.stats[slot].  (pc, pd): capacity and demand
 // of the cell before the warp's first, for lane 0.
 //
 // Level m of the scan adds element ((i >> m) << m) - 1 to the elements i with bit m
@@ -146,16 +190,17 @@ __device__ __forceinline__ double int_to_double(int v) {  // 2^52 + 2^31 + v, le
 // element), 7 between the two passes, and 8 on between warps, each of which adds
 // up the totals it needs in the order of the levels.
 template <int W, int P>
-__device__ __forceinline__ void refresh_track(const GridDev &g, const TrackInfo &ti, const TrackCells<P> &t, float pc,
+__device__ __forceinline__ void refresh_track(const GridDev &g, const TrackWarp &tw, const TrackCells<P> &t, float pc,
                                               float pd, bool vec, int slot) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ double s_total[W];
     __shared__ double s_stage[W][kPassCells];
-    const int n = ti.len, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const TrackInfo &ti = tw.ti;
+    const int n = ti.len, lane = threadIdx.x & 31, warp = tw.warp;
     const double sc = g.short_cost[ti.l];
     const int *elen = ti.dir ? g.ylen : g.xlen;
     const bool evec = (reinterpret_cast<uintptr_t>(elen) & 15) == 0;
-    if (threadIdx.x == 0) atomicAdd(&g.stats[slot], (unsigned long long)n);  // refreshed cells, for the roofline
+    if (tw.leader()) atomicAdd(&g.stats[slot], (unsigned long long)n);  // refreshed cells, for the roofline
     const bool via_float = (double)(float)g.unit_via == g.unit_via;  // then the float sum is the same
     double x[P][4];
     float left_one = 0.f;  // of the cell before this lane's first
@@ -211,12 +256,12 @@ __device__ __forceinline__ void refresh_track(const GridDev &g, const TrackInfo 
         for (int j = 0; j < 4; j++) x[1][j] += o;
     }
     if constexpr (W > 1) {
-        if (lane == 31) s_total[warp] = x[P - 1][3];
+        if (lane == 31) s_total[tw.slot] = x[P - 1][3];
         __syncthreads();
 #pragma unroll
         for (int m = 0; (1 << m) < W; m++) {
             if ((warp >> m) & 1) {
-                const int last = ((warp >> m) << m) - 1;  // the 2^m warps up to it, added up as a tree
+                const int last = tw.slot - warp + ((warp >> m) << m) - 1;  // the 2^m warps up to it, added up as a tree
                 double o[8];
 #pragma unroll
                 for (int k = 0; k < 8; k++) o[k] = k < 1 << m ? s_total[last - k] : 0.0;
@@ -235,7 +280,7 @@ __device__ __forceinline__ void refresh_track(const GridDev &g, const TrackInfo 
 #pragma unroll
     for (int p = 0; p < P; p++) {
         const int i0 = warp * P * kPassCells + p * kPassCells + 4 * lane;
-        store_sums(g.presum + ti.base + i0, n - i0, vec, x[p], s_stage[warp], lane);
+        store_sums(g.presum + ti.base + i0, n - i0, vec, x[p], s_stage[tw.slot], lane);
     }
 }
 
@@ -246,16 +291,17 @@ __device__ __forceinline__ bool track_vec(const GridDev &g, const TrackInfo &ti)
     return ((a | reinterpret_cast<uintptr_t>(g.presum + ti.base) >> 1) & 15) == 0;
 }
 
-template <int W, int P>
-__global__ void __launch_bounds__(32 * W, 28 / W) cost_refresh_kernel(GridDev g, int only_dirty) {
+template <int W, int P, bool MIXED>
+__global__ void __launch_bounds__(32 * W, 28 / W) cost_refresh_kernel(GridDev g, TrackSplit sp, int only_dirty) {
     chain_begin();
-    const int tr = blockIdx.x;
+    TrackWarp tw;
+    if (!own_track<MIXED>(g, sp, tw)) return;
     if (only_dirty) {
-        if (!g.dirty_cost[tr]) return;
+        if (!g.dirty_cost[tw.tr]) return;
     }
-    const TrackInfo ti = decode_track(g, tr);
+    const TrackInfo &ti = tw.ti;
     const bool vec = track_vec(g, ti);
-    const int n = ti.len, lane = threadIdx.x & 31, first = (threadIdx.x >> 5) * P * kPassCells;
+    const int n = ti.len, lane = threadIdx.x & 31, first = tw.warp * P * kPassCells;
     const float *cap = g.cap + ti.base, *dem = g.demand + ti.base;
     TrackCells<P> t;
 #pragma unroll
@@ -266,10 +312,10 @@ __global__ void __launch_bounds__(32 * W, 28 / W) cost_refresh_kernel(GridDev g,
     }
     const bool before = lane == 0 && first > 0 && first <= n;
     const float pc = before ? cap[first - 1] : 0.f, pd = before ? dem[first - 1] : 0.f;
-    refresh_track<W, P>(g, ti, t, pc, pd, vec, 2);
+    refresh_track<W, P>(g, tw, t, pc, pd, vec, 2);
     if (only_dirty) {
         if (W == 1) __syncwarp();  // every lane has seen the flag (warps: refresh_track's barrier)
-        if (threadIdx.x == 0) g.dirty_cost[tr] = 0;
+        if (tw.leader()) g.dirty_cost[tw.tr] = 0;
     }
 }
 
@@ -368,18 +414,21 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
 // beside the cell, a full unit at the track ends), and the costs and prefix
 // sums are rebuilt from the demand in registers.  Tracks with no pending commit
 // and clean costs are skipped.  With refresh = 0 the costs are only marked dirty.
-template <int W, int P>
-__global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev g, int *vcnt, int stamp, int refresh) {
+template <int W, int P, bool MIXED>
+__global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev g, TrackSplit sp, int *vcnt, int stamp,
+                                                                          int refresh) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ int s_sum[W];
-    __shared__ float s_first[W + 1], s_last[W];
+    __shared__ float s_first[W], s_last[W];
     __shared__ long long s_wl[W];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = warp * P * kPassCells;
-    const int tr = blockIdx.x;
     chain_begin();
+    TrackWarp tw;
+    if (!own_track<MIXED>(g, sp, tw)) return;
+    const int lane = threadIdx.x & 31, warp = tw.warp, slot = tw.slot, first = warp * P * kPassCells;
+    const int tr = tw.tr;
     const bool commit = g.dirty_commit[tr] != 0;
     if (!commit && !(refresh && g.dirty_cost[tr])) return;
-    const TrackInfo ti = decode_track(g, tr);
+    const TrackInfo &ti = tw.ti;
     const int n = ti.len;
     const bool vec = track_vec(g, ti);
     float *dem = g.demand + ti.base;
@@ -414,11 +463,11 @@ __global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev 
             for (int j = 0; j < 4; j++) cnt[p][j] += run + inc - sum;
             run += __shfl_sync(kFull, inc, 31);
         }
-        if (lane == 0) s_sum[warp] = run;
+        if (lane == 0) s_sum[slot] = run;
         __syncthreads();
         int base = 0;
 #pragma unroll
-        for (int w = 0; w < W; w++) base += w < warp ? s_sum[w] : 0;
+        for (int w = 0; w < W; w++) base += w < warp ? s_sum[slot - warp + w] : 0;
         // wires: demand, stamps, wirelength; then the vias of cells without this batch's stamp
         long long wl = 0;
         float own[P][4], prev[P][4];  // a via's part of its own edge and of the one before
@@ -439,16 +488,16 @@ __global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev 
                 prev[p][j] = !add || i == 0 ? 0.f : i == n - 1 ? c : 0.5f * c;
             }
         }
-        if (lane == 0) s_first[warp] = prev[0][0];
-        if (tid == 0) s_first[W] = 0.f;
+        if (lane == 0) s_first[slot] = prev[0][0];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) wl += __shfl_down_sync(kFull, wl, o);
-        if (lane == 0) s_wl[warp] = wl;
+        if (lane == 0) s_wl[slot] = wl;
         __syncthreads();
+        const float after = first + P * kPassCells < n ? s_first[slot + 1] : 0.f;  // of the cell after the warp's last
 #pragma unroll
         for (int p = 0; p < P; p++) {
             float next = __shfl_down_sync(kFull, prev[p][0], 1);
-            const float other = p == P - 1 ? s_first[warp + 1] : __shfl_sync(kFull, prev[P - 1][0], 0);
+            const float other = p == P - 1 ? after : __shfl_sync(kFull, prev[P - 1][0], 0);
             if (lane == 31) next = other;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -458,12 +507,12 @@ __global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev 
             const int i0 = first + p * kPassCells + 4 * lane;
             store4(dem + i0, n - i0, vec, t.d[p]);
         }
-        if (lane == 31) s_last[warp] = t.d[P - 1][3];
+        if (lane == 31) s_last[slot] = t.d[P - 1][3];
         __syncthreads();
-        if (lane == 0 && warp > 0) pd = s_last[warp - 1];
-        if (tid == 0) {
+        if (lane == 0 && warp > 0) pd = s_last[slot - 1];
+        if (tw.leader()) {
             long long sum = 0;
-            for (int w = 0; w < W; w++) sum += s_wl[w];
+            for (int w = 0; w * P * kPassCells < n; w++) sum += s_wl[slot + w];
             if (sum) atomicAdd(&g.stats[0], (unsigned long long)sum);
             atomicAdd(&g.stats[3], (unsigned long long)n);  // committed cells, for the roofline
             g.dirty_commit[tr] = 0;
@@ -471,9 +520,9 @@ __global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev 
         }
     } else {
         __syncthreads();
-        if (tid == 0) g.dirty_cost[tr] = 0;
+        if (tw.leader()) g.dirty_cost[tr] = 0;
     }
-    if (refresh) refresh_track<W, P>(g, ti, t, pc, pd, vec, 4);
+    if (refresh) refresh_track<W, P>(g, tw, t, pc, pd, vec, 4);
 }
 
 template <typename T>
@@ -500,7 +549,7 @@ __global__ void track_to_ref_kernel(GridDev g, const T *trk, T *ref) {
 
 }  // namespace
 
-// One CTA per track: the hardware block scheduler hands the dirty tracks to
+// A CTA per track (or per few short ones): the hardware block scheduler hands the dirty tracks to
 // the SMs as they free up, and a CTA that finds its track clean exits at once
 // (a resident grid striding over the tracks balanced the uneven dirty tracks
 // worse: 11.9 -> 15.8 ms per route of the 800k-net design; a resident grid
@@ -525,13 +574,27 @@ static void with_track_shape(int maxlen, F &&f) {
     else with_warps<2, kOnePassCells / (2 * kPassCells) + 1>((maxlen + 2 * kPassCells - 1) / (2 * kPassCells), f);
 }
 
+// Warps and tracks a block for the tracks of either direction, with W warps of P passes a
+// block; returns the grid.
+static dim3 split_tracks(const GridDev &g, int W, int P, TrackSplit &sp) {
+    auto warps = [&](int len) { return (len + P * kPassCells - 1) / (P * kPassCells); };
+    sp.warps0 = warps(g.X);
+    sp.warps1 = warps(g.Y);
+    sp.tracks0 = W / sp.warps0;
+    sp.tracks1 = W / sp.warps1;
+    return dim3(std::max((g.Y + sp.tracks0 - 1) / sp.tracks0, (g.X + sp.tracks1 - 1) / sp.tracks1), g.L);
+}
+
 void launch_cost_refresh(const GridDev &g, bool only_dirty, cudaStream_t s) {
     const int maxlen = g.X > g.Y ? g.X : g.Y;
     const int od = only_dirty ? 1 : 0;
     if (maxlen <= kMaxFusedTrackCells) {
         with_track_shape(maxlen, [&](auto wc, auto pc) {
             constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
-            launch_chained(cost_refresh_kernel<W, P>, dim3(g.ntracks), dim3(32 * W), 0, s, g, od);
+            TrackSplit sp;
+            const dim3 blocks = split_tracks(g, W, P, sp);
+            launch_chained(sp.warps0 == sp.warps1 ? cost_refresh_kernel<W, P, false> : cost_refresh_kernel<W, P, true>,
+                           blocks, dim3(32 * W), 0, s, g, sp, od);
         });
     } else {
         const size_t smem = (size_t)kMaxTrackCells * 8;
@@ -546,7 +609,10 @@ void launch_commit_refresh(const GridDev &g, int *vcnt, int stamp, bool refresh,
     const int rf = refresh ? 1 : 0;
     with_track_shape(maxlen, [&](auto wc, auto pc) {
         constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
-        launch_chained(commit_refresh_kernel<W, P>, dim3(g.ntracks), dim3(32 * W), 0, s, g, vcnt, stamp, rf);
+        TrackSplit sp;
+        const dim3 blocks = split_tracks(g, W, P, sp);
+        launch_chained(sp.warps0 == sp.warps1 ? commit_refresh_kernel<W, P, false> : commit_refresh_kernel<W, P, true>,
+                       blocks, dim3(32 * W), 0, s, g, sp, vcnt, stamp, rf);
     });
 }
 
