@@ -37,8 +37,9 @@ bool pinned_cached(size_t bytes);
 
 // Copies to and from the caller's pageable memory by several host threads
 // through page-locked chunks (host_copy.cpp), after the work queued on `s`.
-// copy_to_host returns when dst is complete; the others when src may be reused
-// (the last one rounds to BF16 on the way).
+// copy_to_host returns when dst is complete; the others when src may be reused, but for
+// a page-locked src of copy_to_device, which is in use until the copy has run (the last
+// one rounds to BF16 on the way).
 void copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s);
 void copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t s);
 void copy_to_device_bf16(__nv_bfloat16 *dst, const float *src, size_t n, cudaStream_t s);

@@ -1,0 +1,41 @@
+"""Copies of results and inputs between the device and the caller's memory, of each
+kind that memory can be."""
+import time
+
+import numpy as np
+import pytest
+
+import instantgr_b200 as ig
+
+pytestmark = pytest.mark.gpu
+
+
+def _least(f, n=40):
+    best = 1e9
+    for _ in range(n):
+        t0 = time.perf_counter()
+        f()
+        best = min(best, time.perf_counter() - t0)
+    return best
+
+
+def test_page_locked_memory_is_copied_directly(tmp_path):
+    """Demand of 9 MB into a page-locked array: the copy itself (178 us) with a layout
+    kernel and the wait around it (20 us), so 1.6 times a plain copy at most; through
+    staging chunks and threads it took 2.3 times at the least."""
+    import torch
+    X, Y = 420, 600
+    cap, net = str(tmp_path / "d.cap"), str(tmp_path / "d.net")
+    ig.generate_custom(X, Y, 2000, seed=1, cap=cap, net=net)
+    r = ig.Router(cap, net, rrr_iters=0)
+    r.run()
+    want = r.demand()
+    locked = torch.full((9 * X * Y,), -1.0).pin_memory()
+    get = lambda: ig._check(ig.lib().igr_router_demand(r.h, locked.numpy()))  # noqa: E731
+    get()
+    assert np.array_equal(locked.numpy(), want)
+    mine = _least(get)
+    dev = torch.from_numpy(want).cuda()
+    plain = _least(lambda: (locked.copy_(dev), torch.cuda.synchronize()))
+    r.close()
+    assert mine <= 1.6 * plain, (mine, plain)
