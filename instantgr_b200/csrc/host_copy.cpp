@@ -9,6 +9,8 @@
 // features rounded to BF16 on the way up, 164 MB down, 16 cores) went from 95 ms
 // to 11; with 8 threads 13, with 4 threads 20.  Below kMinBytes the threads cost
 // more than they save.
+#include <sched.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -26,6 +28,13 @@ namespace {
 constexpr size_t kChunk = (size_t)1 << 20;
 constexpr size_t kMinBytes = (size_t)4 << 20;
 constexpr int kMaxThreads = 16;
+
+// Cores this process may run on (the machine's number of them says nothing about that).
+int usable_cores() {
+    cpu_set_t set;
+    if (sched_getaffinity(0, sizeof set, &set) != 0) return hw_threads();
+    return std::max(1, CPU_COUNT(&set));
+}
 
 // fn(worker) on `n` threads (the caller's among them), each on the caller's
 // device; the first exception is rethrown once all have returned
@@ -85,7 +94,7 @@ struct Slot {
 template <typename F>
 void by_chunks(size_t items, size_t size, cudaStream_t s, F &&each) {
     const size_t per = kChunk / size, chunks = (items + per - 1) / per;
-    const int n = (int)std::min<size_t>({(size_t)kMaxThreads, (size_t)std::max(1, hw_threads()), chunks});
+    const int n = (int)std::min<size_t>({(size_t)kMaxThreads, (size_t)usable_cores(), chunks});
     std::atomic<size_t> next{0};
     std::atomic<bool> stop{false};
     run_workers(n, [&](int) {
@@ -108,11 +117,14 @@ void by_chunks(size_t items, size_t size, cudaStream_t s, F &&each) {
     });
 }
 
-// Whether the driver copies to and from p without staging: page-locked or registered
-// memory.  A copy of it through the chunks would move everything twice (34 MB of demand
-// in 1.29 ms, directly in 0.67).  What is not plain host memory at all is left to the
-// driver too.
+// Whether a copy to or from p is best left to the driver.  Page-locked or registered
+// memory needs no staging: through the chunks everything would move twice (34 MB of
+// demand in 1.29 ms, directly in 0.67).  What is not plain host memory at all is the
+// driver's to judge.  And where there is no second core, its own staging is faster than
+// a thread that waits for each chunk (34 MB into an array in use: 2.2 ms, in chunks by
+// as many threads as the machine has cores 3.7; with two cores and two threads 1.7).
 bool direct(const void *p) {
+    if (usable_cores() < 2) return true;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();

@@ -1,11 +1,14 @@
 """Copies of results and inputs between the device and the caller's memory, of each
 kind that memory can be."""
+import subprocess
+import sys
 import time
 
 import numpy as np
 import pytest
 
 import instantgr_b200 as ig
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +42,35 @@ def test_page_locked_memory_is_copied_directly(tmp_path):
     plain = _least(lambda: (locked.copy_(dev), torch.cuda.synchronize()))
     r.close()
     assert mine <= 1.6 * plain, (mine, plain)
+
+
+ONE_CORE = """
+import os, sys, time
+os.sched_setaffinity(0, {min(os.sched_getaffinity(0))})
+sys.path.insert(0, sys.argv[1])
+import numpy as np, torch
+import instantgr_b200 as ig
+X, Y = 840, 1140
+cap, net = sys.argv[2] + "/d.cap", sys.argv[2] + "/d.net"
+ig.generate_custom(X, Y, 2000, seed=1, cap=cap, net=net)
+r = ig.Router(cap, net, rrr_iters=0)
+r.run()
+out, dev = torch.zeros(9 * X * Y), torch.zeros(9 * X * Y, device="cuda")
+def least(f):
+    t = []
+    for _ in range(20):
+        a = time.perf_counter(); f(); t.append(time.perf_counter() - a)
+    return min(t[2:])
+mine = least(lambda: ig._check(ig.lib().igr_router_demand(r.h, out.numpy())))
+plain = least(lambda: (out.copy_(dev), torch.cuda.synchronize()))
+print(mine / plain)
+"""
+
+
+def test_one_core_copies_as_the_driver_does(tmp_path):
+    """34 MB into plain memory by a process of one core: the driver's copy and the layout
+    kernel, so at most 1.35 times the driver's copy alone; chunk by chunk it took 1.7."""
+    p = subprocess.run([sys.executable, "-c", ONE_CORE, ROOT, str(tmp_path)], capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
+    assert float(p.stdout.split()[-1]) <= 1.35
