@@ -16,6 +16,7 @@
 #include <cstring>
 #include <exception>
 #include <mutex>
+#include <string>
 #include <thread>
 #include <vector>
 
@@ -36,17 +37,51 @@ int usable_cores() {
     return std::max(1, CPU_COUNT(&set));
 }
 
-// fn(worker) on `n` threads (the caller's among them), each on the caller's
-// device; the first exception is rethrown once all have returned
+// The caller's CUDA context, for its workers.  It need not be the primary one of its
+// device, which cudaSetDevice would take: events of that one are refused on a stream of
+// another.
+class CallerContext {
+    int (*set_)(void *) = nullptr;
+    void *ctx_ = nullptr;
+
+    template <typename F>
+    static void entry(const char *name, F &f) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        cuda_check(cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q), name);
+        if (q != cudaDriverEntryPointSuccess || !p) throw Error(ERR_CUDA, std::string("no driver entry point ") + name);
+        f = reinterpret_cast<F>(p);
+    }
+
+public:
+    CallerContext() {
+        int (*get)(void **);
+        entry("cuCtxGetCurrent", get);
+        entry("cuCtxSetCurrent", set_);
+        int rc = get(&ctx_);
+        if (rc == 0 && !ctx_) {  // a thread that has not used CUDA yet: its device's primary context
+            int dev = 0;
+            cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+            cuda_check(cudaSetDevice(dev), "cudaSetDevice");
+            rc = get(&ctx_);
+        }
+        if (rc != 0) throw Error(ERR_CUDA, "cuCtxGetCurrent");
+    }
+    void take() const {
+        if (set_(ctx_) != 0) throw Error(ERR_CUDA, "cuCtxSetCurrent");
+    }
+};
+
+// fn(worker) on `n` threads (the caller's among them), each in the caller's
+// context; the first exception is rethrown once all have returned
 template <typename F>
 void run_workers(int n, F &&fn) {
-    int dev = 0;
-    cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    const CallerContext caller;
     std::mutex mu;
     std::exception_ptr err;
     auto work = [&](int w) {
         try {
-            if (w > 0) cuda_check(cudaSetDevice(dev), "cudaSetDevice");
+            if (w > 0) caller.take();
             fn(w);
         } catch (...) {
             std::lock_guard<std::mutex> lock(mu);
@@ -54,10 +89,11 @@ void run_workers(int n, F &&fn) {
         }
     };
     std::vector<std::thread> ts;
+    ts.reserve((size_t)n);  // no exception may leave this function past a running thread
     for (int w = 1; w < n; w++) {
         try {
             ts.emplace_back(work, w);
-        } catch (const std::system_error &) {
+        } catch (const std::exception &) {
             break;  // fewer threads than asked for: the others take the chunks
         }
     }

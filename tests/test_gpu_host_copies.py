@@ -74,3 +74,40 @@ def test_one_core_copies_as_the_driver_does(tmp_path):
                        timeout=300)
     assert p.returncode == 0, p.stderr[-2000:]
     assert float(p.stdout.split()[-1]) <= 1.35
+
+
+OWN_CONTEXT = """
+import ctypes, sys
+sys.path.insert(0, sys.argv[1])
+if sys.argv[2] == "own":
+    cu, ctx, dev = ctypes.CDLL("libcuda.so.1"), ctypes.c_void_p(), ctypes.c_int()
+    assert cu.cuInit(0) == 0 and cu.cuDeviceGet(ctypes.byref(dev), 0) == 0
+    assert cu.cuCtxCreate_v2(ctypes.byref(ctx), 0, dev) == 0
+import hashlib
+import numpy as np
+import instantgr_b200 as ig
+m = ig.Seed.load()
+for X in (100, 400):
+    print(hashlib.sha256(m.predict(np.random.default_rng(1).random((X, X, 16), np.float32)).tobytes()).hexdigest())
+if sys.argv[2] == "thread":  # the first use of CUDA by its thread is a copy in chunks
+    import threading
+    m.set_tile(144, 16)
+    x = np.random.default_rng(2).random((6, 144, 144, 16), np.float32)
+    want, got = m.grad(x, x)[0], []
+    t = threading.Thread(target=lambda: got.append(m.grad(x, x)[0]))
+    t.start(); t.join()
+    assert abs(got[0] - want) <= 1e-12 * want
+m.close()
+"""
+
+
+def test_predictions_in_a_context_of_the_callers_own():
+    """Inputs and results below and above the staging limit, in a process whose
+    CUDA context is not the device's primary one: the primary one's predictions.
+    (The loss of a second thread's call: sums of 1.2M squares in 64 bits, in any order.)"""
+    out = []
+    for kind in ("thread", "own"):
+        p = subprocess.run([sys.executable, "-c", OWN_CONTEXT, ROOT, kind], capture_output=True, text=True, timeout=300)
+        assert p.returncode == 0, p.stderr[-2000:]
+        out.append(p.stdout)
+    assert out[0] == out[1]
