@@ -986,7 +986,10 @@ void Router::phase1() {
 // from medium nets, or one class of all nets, by timing the phase-1 batch loop
 // of this design once per candidate (the routes are the same for every
 // candidate).  Results are cached per grid and net count in
-// $IGR_TUNE_CACHE (default ~/.cache/instantgr_b200/tune.txt).
+// $IGR_TUNE_CACHE (default ~/.cache/instantgr_b200/tune.txt), a line
+// "dp2 X Y nets batches classes split" each; the tag is that of the tree DP's kernel
+// and its launches, so that lines timed with other ones are not taken.
+constexpr char kTuneTag[] = "dp2";
 static std::string tune_cache_path() {
     if (const char *p = std::getenv("IGR_TUNE_CACHE")) return p;
     const char *h = std::getenv("HOME");
@@ -996,21 +999,18 @@ static std::string tune_cache_path() {
 void Router::autotune(int nb) {
     const int R = (int)ns.nets.size();
     char key[96];
-    std::snprintf(key, sizeof key, "%d %d %d %d", ns.X, ns.Y, R, nb);
+    std::snprintf(key, sizeof key, "%s %d %d %d %d", kTuneTag, ns.X, ns.Y, R, nb);
     const std::string path = tune_cache_path();
     if (FILE *f = std::fopen(path.c_str(), "r")) {
         char line[256];
         while (std::fgets(line, sizeof line, f)) {
-            int x, y, r, b, cl, sp, l0, l1, l2;
-            if (std::sscanf(line, "%d %d %d %d %d %d %d %d %d", &x, &y, &r, &b, &cl, &sp, &l0, &l1, &l2) == 9) {
-                char k2[96];
-                std::snprintf(k2, sizeof k2, "%d %d %d %d", x, y, r, b);
-                auto lanes_ok = [](int l) { return l == 16 || l == 32; };
-                if (std::string(k2) == key && (cl == 1 || cl == 3) && sp >= 1 && sp <= 6 && lanes_ok(l0) &&
-                    lanes_ok(l1) && lanes_ok(l2)) {
-                    tune.classes = cl; tune.split = sp;
-                    tuned = true;
-                }
+            int cl, sp;
+            const size_t n = std::strlen(key);
+            if (std::strncmp(line, key, n) != 0 || line[n] != ' ') continue;
+            if (std::sscanf(line + n, "%d %d", &cl, &sp) == 2 && (cl == 1 || cl == 3) && sp >= 1 && sp <= 6) {
+                tune.classes = cl;
+                tune.split = sp;
+                tuned = true;
             }
         }
         std::fclose(f);
@@ -1060,7 +1060,7 @@ void Router::autotune(int nb) {
             if (i == dir.size() || dir[i] == '/') (void)mkdir(dir.substr(0, i).c_str(), 0755);
     }
     if (FILE *f = std::fopen(path.c_str(), "a")) {
-        std::fprintf(f, "%s %d %d 32 32 32\n", key, tune.classes, tune.split);  // 32 lanes per net in each class
+        std::fprintf(f, "%s %d %d\n", key, tune.classes, tune.split);
         std::fclose(f);
     }
 }
