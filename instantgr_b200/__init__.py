@@ -579,7 +579,8 @@ class Seed:
 
     def predict(self, features) -> np.ndarray:
         f = np.ascontiguousarray(features, dtype=np.float32)
-        out = np.empty_like(f)  # written in full
+        # written in full, but where a GCell has more than the 16 channels that there are
+        out = np.empty_like(f) if f.shape[2:] == (16,) else np.zeros_like(f)
         self._c(lib().igr_seed_predict(self.h, f.shape[0], f.shape[1], f.reshape(-1), out.reshape(-1)))
         return out
 
