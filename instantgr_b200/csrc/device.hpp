@@ -100,7 +100,8 @@ struct TreeBatchDev {
 };
 // scratch per node of a net of more than kPatternNodeTile nodes: 45 range costs
 // (doubles), then 8 unused ints, 45 backtrace codes (shorts, padded to 23 ints),
-// the chosen range and 4 unused ints
+// the chosen range and 4 unused ints (left over from an earlier kernel; the limits of
+// the allocation-free entry follow from this size, so it stays)
 constexpr int kPatternScratchD = 45, kPatternScratchI = 8 + 23 + 1 + 4;
 // doubles of scratch needed for `nodes` nodes of nets kept in global memory
 inline int64_t pattern_scratch_doubles(int64_t nodes) {

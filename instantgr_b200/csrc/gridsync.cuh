@@ -22,7 +22,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // `epoch` is a per-thread register starting at 0, advanced identically by
-// every thread of the block.  Returns false on timeout or a reported error.
+// every thread of the block.  Returns false when this block's wait, or another's, ran out.
 // `limit_ns` bounds the wait; `phantom` (a test hook, normally 0) adds
 // arrivals that never come, so that the wait runs out by construction.
 __device__ __forceinline__ bool grid_sync(unsigned long long *count, int *err, unsigned long long &epoch,

@@ -1,8 +1,8 @@
 // Learned congestion seed: a small BF16 convolutional encoder-decoder that
 // predicts per-layer routing demand from placement features, trained on the
-// demand maps the plain router produces.  Device kernels in seed_nn.cu
-// (tcgen05 implicit-GEMM convolutions, TMEM accumulators), host model in
-// seed_model.cpp.  It has no counterpart in InstantGR.
+// demand maps the plain router produces.  Device kernels in seed_conv.cu
+// (tcgen05 implicit-GEMM convolutions, TMEM accumulators) and seed_nn.cu, host
+// model in seed_model.cpp.  It has no counterpart in InstantGR.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

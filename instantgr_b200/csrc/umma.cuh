@@ -23,9 +23,6 @@ __device__ __forceinline__ unsigned long long now_ns() {
     return t;
 }
 
-// element offset of (row r, k) in a 128 (or fewer) x 16 sub-tile
-__device__ __forceinline__ int sub_idx(int r, int k) { return (r >> 3) * 128 + (k >> 3) * 64 + (r & 7) * 8 + (k & 7); }
-
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lead, uint32_t stride) {
     uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFF);  // start address
     d |= (uint64_t)(lead >> 4) << 16;                // leading byte offset
@@ -33,7 +30,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lead, uin
     d |= (uint64_t)1 << 46;                          // descriptor version of sm_100
     return d;                                        // base offset 0, no swizzle
 }
-// the sub-tiles of sub_idx: K halves 128 bytes apart, 8-row groups 256
+// a sub-tile of 16 K columns and 128 (or fewer) rows, end to end: per group of 8 rows
+// the core matrices of its two K halves, 128 bytes apart, groups 256
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) { return smem_desc(saddr, 128, 256); }
 
 // kind::f16 instruction descriptor: F32 accumulator, BF16 A and B, both K-major
@@ -130,18 +128,8 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
                  : "memory");
 }
 
-// 8 consecutive f32 columns of this thread's TMEM lane (warp w reads lanes 32w..32w+31)
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = __uint_as_float(r[j]);
-}
-
-// 16 or 32 consecutive f32 columns of this thread's TMEM lane, to be waited for with tmem_wait
+// 16 consecutive f32 columns of this thread's TMEM lane (warp w reads lanes 32 (w % 4) on),
+// to be waited for with tmem_wait
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
                  "[%16];"
