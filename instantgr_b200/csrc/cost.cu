@@ -115,6 +115,7 @@ constexpr int kOnePassCells = 1024;  // tracks of at most this many cells: one p
 struct TrackSplit {
     int warps0, warps1;    // per track, of the layers along x and along y
     int tracks0, tracks1;  // per block
+    int blocks0, blocks1;  // per layer
 };
 // this warp's track and its number among the track's warps and the block's
 struct TrackWarp {
@@ -122,23 +123,28 @@ struct TrackWarp {
     int tr, warp, slot;
     __device__ __forceinline__ bool leader() const { return warp == 0 && (threadIdx.x & 31) == 0; }
 };
-// blocks x: of a layer, y: layer; false: no track for this warp.  MIXED: some tracks take
+// The blocks are in the order of the layers.  False: no track for this warp.  MIXED: some tracks take
 // fewer warps than the block has (none does at 1600 x 1600: 170 us a call without this, 174 with it).
 template <bool MIXED>
 __device__ __forceinline__ bool own_track(const GridDev &g, const TrackSplit &sp, TrackWarp &tw) {
-    const int l = blockIdx.y, dir = layer_dir(g, l);
-    int t = blockIdx.x;
+    const int first = g.DIR ? sp.blocks1 : sp.blocks0, pair = sp.blocks0 + sp.blocks1;
+    int l = 0, t = blockIdx.x;  // layer and block of it, two layers at a time
+    for (; t >= pair; t -= pair) l += 2;
+    if (t >= first) {
+        t -= first;
+        l++;
+    }
+    const int dir = layer_dir(g, l);
     if constexpr (MIXED) {
         const int warps = dir ? sp.warps1 : sp.warps0, tracks = dir ? sp.tracks1 : sp.tracks0;
         tw.slot = tw.warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // shuffled: uniform, for the compiler
         int group = 0;
         for (; tw.warp >= warps; tw.warp -= warps) group++;
-        if (group >= tracks) return false;
         t = t * tracks + group;
+        if (group >= tracks || t >= (dir ? g.X : g.Y)) return false;
     } else {
         tw.slot = tw.warp = threadIdx.x >> 5;
     }
-    if (t >= (dir ? g.X : g.Y)) return false;
     tw.tr = (l >> 1) * (g.X + g.Y) + (l & 1) * (g.DIR ? g.X : g.Y) + t;
     tw.ti.l = l;
     tw.ti.t = t;
@@ -575,14 +581,17 @@ static void with_track_shape(int maxlen, F &&f) {
 }
 
 // Warps and tracks a block for the tracks of either direction, with W warps of P passes a
-// block; returns the grid.
-static dim3 split_tracks(const GridDev &g, int W, int P, TrackSplit &sp) {
+// block; returns the number of blocks.
+static int split_tracks(const GridDev &g, int W, int P, TrackSplit &sp) {
     auto warps = [&](int len) { return (len + P * kPassCells - 1) / (P * kPassCells); };
     sp.warps0 = warps(g.X);
     sp.warps1 = warps(g.Y);
     sp.tracks0 = W / sp.warps0;
     sp.tracks1 = W / sp.warps1;
-    return dim3(std::max((g.Y + sp.tracks0 - 1) / sp.tracks0, (g.X + sp.tracks1 - 1) / sp.tracks1), g.L);
+    sp.blocks0 = (g.Y + sp.tracks0 - 1) / sp.tracks0;
+    sp.blocks1 = (g.X + sp.tracks1 - 1) / sp.tracks1;
+    const int odd = g.L / 2, even = g.L - odd;  // layers of the other and of layer 0's direction
+    return g.DIR ? even * sp.blocks1 + odd * sp.blocks0 : even * sp.blocks0 + odd * sp.blocks1;
 }
 
 void launch_cost_refresh(const GridDev &g, bool only_dirty, cudaStream_t s) {
@@ -592,9 +601,9 @@ void launch_cost_refresh(const GridDev &g, bool only_dirty, cudaStream_t s) {
         with_track_shape(maxlen, [&](auto wc, auto pc) {
             constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
             TrackSplit sp;
-            const dim3 blocks = split_tracks(g, W, P, sp);
+            const int blocks = split_tracks(g, W, P, sp);
             launch_chained(sp.warps0 == sp.warps1 ? cost_refresh_kernel<W, P, false> : cost_refresh_kernel<W, P, true>,
-                           blocks, dim3(32 * W), 0, s, g, sp, od);
+                           dim3(blocks), dim3(32 * W), 0, s, g, sp, od);
         });
     } else {
         const size_t smem = (size_t)kMaxTrackCells * 8;
@@ -610,9 +619,9 @@ void launch_commit_refresh(const GridDev &g, int *vcnt, int stamp, bool refresh,
     with_track_shape(maxlen, [&](auto wc, auto pc) {
         constexpr int W = decltype(wc)::value, P = decltype(pc)::value;
         TrackSplit sp;
-        const dim3 blocks = split_tracks(g, W, P, sp);
+        const int blocks = split_tracks(g, W, P, sp);
         launch_chained(sp.warps0 == sp.warps1 ? commit_refresh_kernel<W, P, false> : commit_refresh_kernel<W, P, true>,
-                       blocks, dim3(32 * W), 0, s, g, sp, vcnt, stamp, rf);
+                       dim3(blocks), dim3(32 * W), 0, s, g, sp, vcnt, stamp, rf);
     });
 }
 
