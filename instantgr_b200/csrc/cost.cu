@@ -123,10 +123,16 @@ struct TrackWarp {
     int tr, warp, slot;
     __device__ __forceinline__ bool leader() const { return warp == 0 && (threadIdx.x & 31) == 0; }
 };
-// The blocks are in the order of the layers.  False: no track for this warp.  MIXED: some tracks take
-// fewer warps than the block has (none does at 1600 x 1600: 170 us a call without this, 174 with it).
+// The blocks are in the order of the layers.  False: no track for this warp.  MIXED: some
+// tracks take fewer warps than the block has (none does at 1600 x 1600: 167 us a call without
+// this, 174 with it; then a block is a track, whose flags are read before anything else).
 template <bool MIXED>
 __device__ __forceinline__ bool own_track(const GridDev &g, const TrackSplit &sp, TrackWarp &tw) {
+    if constexpr (!MIXED) {
+        tw.tr = blockIdx.x;
+        tw.slot = tw.warp = threadIdx.x >> 5;
+        return true;
+    }
     const int first = g.DIR ? sp.blocks1 : sp.blocks0, pair = sp.blocks0 + sp.blocks1;
     int l = 0, t = blockIdx.x;  // layer and block of it, two layers at a time
     for (; t >= pair; t -= pair) l += 2;
@@ -135,16 +141,12 @@ __device__ __forceinline__ bool own_track(const GridDev &g, const TrackSplit &sp
         l++;
     }
     const int dir = layer_dir(g, l);
-    if constexpr (MIXED) {
-        const int warps = dir ? sp.warps1 : sp.warps0, tracks = dir ? sp.tracks1 : sp.tracks0;
-        tw.slot = tw.warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // shuffled: uniform, for the compiler
-        int group = 0;
-        for (; tw.warp >= warps; tw.warp -= warps) group++;
-        t = t * tracks + group;
-        if (group >= tracks || t >= (dir ? g.X : g.Y)) return false;
-    } else {
-        tw.slot = tw.warp = threadIdx.x >> 5;
-    }
+    const int warps = dir ? sp.warps1 : sp.warps0, tracks = dir ? sp.tracks1 : sp.tracks0;
+    tw.slot = tw.warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // shuffled: uniform, for the compiler
+    int group = 0;
+    for (; tw.warp >= warps; tw.warp -= warps) group++;
+    t = t * tracks + group;
+    if (group >= tracks || t >= (dir ? g.X : g.Y)) return false;
     tw.tr = (l >> 1) * (g.X + g.Y) + (l & 1) * (g.DIR ? g.X : g.Y) + t;
     tw.ti.l = l;
     tw.ti.t = t;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(32 * W, 28 / W) cost_refresh_kernel(GridDev g,
     if (only_dirty) {
         if (!g.dirty_cost[tw.tr]) return;
     }
+    if (!MIXED) tw.ti = decode_track(g, tw.tr);
     const TrackInfo &ti = tw.ti;
     const bool vec = track_vec(g, ti);
     const int n = ti.len, lane = threadIdx.x & 31, first = tw.warp * P * kPassCells;
@@ -434,6 +437,7 @@ __global__ void __launch_bounds__(32 * W, 28 / W) commit_refresh_kernel(GridDev 
     const int tr = tw.tr;
     const bool commit = g.dirty_commit[tr] != 0;
     if (!commit && !(refresh && g.dirty_cost[tr])) return;
+    if (!MIXED) tw.ti = decode_track(g, tr);
     const TrackInfo &ti = tw.ti;
     const int n = ti.len;
     const bool vec = track_vec(g, ti);
