@@ -107,8 +107,8 @@ constexpr int kOnePassCells = 1024;  // tracks of at most this many cells: one p
 // A block has the warps that a track of the longer direction needs; of the other
 // direction it takes as many tracks as fit, each with the warps it needs.  (With a
 // block per track of either, the others' warps evaluated the cost model for cells that
-// are not there: 64 x 4096 cells took 645 us a call, 2000 x 200 136, now 85 and 57;
-// 840 x 1140, where that was one of the five warps of every second layer, 92 and 87.)
+// are not there: 64 x 4096 cells took 645 us a call, 2000 x 200 136, now 81 and 59;
+// 840 x 1140, where that was one of the five warps of every second layer, 92 and 85.)
 // Tracks of a block share its barriers, though they need not come to the same number
 // of them: a warp without a track, or done with it, leaves the kernel, and a barrier waits
 // for the threads still in it.
