@@ -96,9 +96,9 @@ __device__ __forceinline__ void unit_costs(float c, float d, double sc, float &o
 // passes, four consecutive ones a lane and pass, so that whole sectors are read and
 // written where tracks start on 16 bytes, two levels of the scan are within a lane,
 // and the block has one barrier.  Bound by the instructions of the cost model
-// (81% of the issue slots; 9 of about 150 per cell go to the slowest pipe,
+// (79% of the issue slots; 9 of about 150 per cell go to the slowest pipe,
 // exponentials and conversions).  1600 x 1600 cells, 9 layers: 153 us; 840 x 1140:
-// 72; as rows of 256 cells with the costs in shared memory and ten barriers a track
+// 63; as rows of 256 cells with the costs in shared memory and ten barriers a track
 // 185 and 81.  (Predicated additions in the scan, end cells apart from the others
 // and a path for cells with capacity alone took fewer instructions but 164 to 172 us.)
 constexpr int kPassCells = 128;
